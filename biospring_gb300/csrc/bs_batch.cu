@@ -96,7 +96,9 @@ __global__ void __launch_bounds__(kBatchBboxBlock) k_batch_bbox(Params p)
         g.radius = p.list_radius / static_cast<float>(kSparseDiv);
         int nc[3] = {1, 1, 1};
         double gmin[3] = {0.0, 0.0, 0.0};
-        double cells = ok ? grid_dims(mn, mx, g.radius, gmin, nc) : 1.0;
+        double cells = !ok           ? 1.0
+                       : p.lists_off ? free_grid_dims(mn, mx, g.radius, free_cells(n1 - n0), gmin, nc)
+                                     : grid_dims(mn, mx, g.radius, gmin, nc);
         if (!(cells <= static_cast<double>(kMaxSysCells)))
         {
             // one cell holds the whole system: the neighbour walk sees every particle, which

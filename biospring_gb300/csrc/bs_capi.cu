@@ -1160,17 +1160,16 @@ int bs_setup(bs_sim *s, const bs_config *cfg)
         if (on[t])
             list_radius = std::max(list_radius, R);
     }
-    if (!(on[0] || on[1] || on[2] || on[3]))
-        list_radius = 1.0e4; // no nonbonded term: a grid of a few cells keeps the rebuild trivial
-    p.list_radius = static_cast<float>(list_radius);
+    p.lists_off = on[0] || on[1] || on[2] || on[3] ? 0 : 1;
     // grid cells and density from the bounding box of each system (one system unless batched)
     const int nsys = batch ? static_cast<int>(s->sys_off.size() - 1) : 1;
     // cells of the list radius (warp-per-particle build, batches) and of a kGridDiv-th of it
     // (cell-block build)
-    double cells1 = 0.0, cells_div = 0.0, density = 0.0;
+    double cells1 = 0.0, cells_div = 0.0, density = 0.0, free_total = 0.0;
     for (int b = 0; b < nsys; ++b)
     {
         const int64_t i0 = batch ? s->sys_off[b] : 0, i1 = batch ? s->sys_off[b + 1] : n;
+        free_total += free_cells(static_cast<double>(i1 - i0));
         double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
         for (int64_t i = i0; i < i1; ++i)
             for (int k = 0; k < 3; ++k)
@@ -1193,7 +1192,15 @@ int bs_setup(bs_sim *s, const bs_config *cfg)
     // faster than one block per (mostly empty) group of cells
     p.pl_sparse = static_cast<double>(n) < 8.0 * cells1 ? 1 : 0;
     const double cells = batch || p.pl_sparse ? cells1 : cells_div;
-    const int cell_cap = static_cast<int>(std::min(2.0 * cells + 1024.0, 2.0e8));
+    int cell_cap = static_cast<int>(std::min(2.0 * cells + 1024.0, 2.0e8));
+    if (p.lists_off)
+    {
+        // no nonbonded term: cells of about kFreeCell particles at the densest system's density
+        list_radius = std::min(std::max(std::cbrt(kFreeCell / density), 1e-3), 1.0e4);
+        p.pl_sparse = 1;
+        cell_cap = static_cast<int>(std::min(free_total + 1024.0, 1.0e9));
+    }
+    p.list_radius = static_cast<float>(list_radius);
     // first capacity: 1.5x the mean count expected in the list sphere, at least 32
     int caps[kLists];
     for (int t = 0; t < kLists; ++t)

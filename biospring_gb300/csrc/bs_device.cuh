@@ -99,6 +99,22 @@ __device__ __forceinline__ double grid_dims(const float (&mn)[3], const float (&
     return cells;
 }
 
+// Grid of a system without nonbonded terms (Params::lists_off). No pair is looked for, the cells only
+// give the particles a spatial order, so the edge is free: it starts at the host's choice (about
+// kFreeCell particles a cell) and doubles until the box fits `most` cells, so that a system may
+// spread without limit.
+__device__ __forceinline__ double free_grid_dims(const float (&mn)[3], const float (&mx)[3], float &edge, double most,
+                                                 double (&gmin)[3], int (&nc)[3])
+{
+    double cells = grid_dims(mn, mx, edge, gmin, nc);
+    for (int it = 0; it < 128 && !(cells <= most); ++it)
+    {
+        edge *= 2.0f;
+        cells = grid_dims(mn, mx, edge, gmin, nc);
+    }
+    return cells;
+}
+
 // Exact reference test of one candidate pair for one cutoff: the grid filter compares the FP64
 // distance of the float coordinates (nsearch.hpp:230, measure.hpp:163-169); the force routine
 // then compares the float-rounded FP64 norm of the float difference vector (Particle.cpp:222-224,

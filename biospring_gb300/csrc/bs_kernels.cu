@@ -106,10 +106,11 @@ __global__ void __launch_bounds__(kBboxBlock) k_bbox(Params p)
     }
     // the cell-block list build uses cells of a kGridDiv-th of the list radius, the warp-per-particle
     // build (sparse systems) cells of the list radius
-    const float edge = p.list_radius / static_cast<float>(p.pl_sparse ? kSparseDiv : kGridDiv);
+    float edge = p.list_radius / static_cast<float>(p.pl_sparse ? kSparseDiv : kGridDiv);
     int nc[3];
     double gmin[3];
-    const double cells = grid_dims(mn, mx, edge, gmin, nc);
+    const double cells = p.lists_off ? free_grid_dims(mn, mx, edge, free_cells(p.n), gmin, nc)
+                                     : grid_dims(mn, mx, edge, gmin, nc);
     for (int k = 0; k < 3; ++k)
         ctl->gmin[k] = gmin[k];
     ctl->gradius = edge;
@@ -1242,6 +1243,8 @@ int launch_rebuild(const Params &p, cudaStream_t st)
                  static_cast<unsigned>((static_cast<long long>(p.npad) * p.ell_lanes + kBuildBlock - 1) / kBuildBlock),
                  kBuildBlock, 0, st, p);
     launched += 4;
+    if (p.lists_off)
+        return launched;
     if (p.nsys > 0 || p.pl_sparse)
         return launched + launch_batch_pairlist(p, st);
     // one block per group of kGridDiv^3 cells (the grid's size is only known on the device: cover
