@@ -35,8 +35,12 @@ namespace
 {
 
 constexpr int kNaMaxN = BS_NOALLOC_MAX_PARTICLES;
-constexpr int kNaBlock = 64;                         // threads per block, one particle each
-constexpr int kNaMaxBlocks = kNaMaxN / kNaBlock;     // 256
+constexpr int kNaBlock = 256;                        // threads per block
+constexpr int kNaHomes = 4;                          // home particles of a warp
+constexpr int kNaMaxSplit = kNaBlock / 32;           // most warps that share a group of homes
+// most blocks of a call: 4, 8 and 16 homes a block up to 5,000, 10,000 and kNaMaxN particles
+// (na_split): at most 1,250
+constexpr int kNaMaxBlocks = 1280;
 constexpr int kNaTerms = 3;                          // steric, Coulomb, hydrophobic
 
 // Scratch layout (byte offsets into na_scratch):
@@ -49,7 +53,7 @@ constexpr size_t kNaPosOff = 0;
 constexpr size_t kNaPrmOff = kNaPosOff + sizeof(float4) * kNaMaxN;
 constexpr size_t kNaBlkOff = kNaPrmOff + sizeof(float4) * kNaMaxN;
 constexpr size_t kNaDoneOff = kNaBlkOff + sizeof(double) * kNaMaxBlocks * kNaTerms;
-constexpr size_t kNaBytes = (kNaDoneOff + sizeof(unsigned int) + 255) / 256 * 256; // 518 KB
+constexpr size_t kNaBytes = (kNaDoneOff + sizeof(unsigned int) + 255) / 256 * 256; // 555 KB
 
 static __device__ __align__(256) unsigned char na_scratch[kNaBytes];
 
@@ -126,6 +130,7 @@ __global__ void __launch_bounds__(256) k_na_pack(NaParams p, const float *__rest
                                                  const float *__restrict__ hydro,
                                                  const uint8_t *__restrict__ is_static, NaBuffers b)
 {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= p.n)
         return;
@@ -157,149 +162,264 @@ __global__ void __launch_bounds__(256) k_na_pack(NaParams p, const float *__rest
     b.prm[i] = make_float4(static_cast<float>(F), q, h, __uint_as_float(fl));
 }
 
-// One thread per particle i; all particles j stream through shared memory in tiles of
-// kNaBlock. Energies: FP32 per thread, FP64 per block, summed in block order by the last block.
-__global__ void __launch_bounds__(kNaBlock) k_na_forces(NaParams p, float *__restrict__ forces,
+// All-pairs forces in two phases a warp. A warp owns kNaHomes home particles and runs through its
+// share of the particles j, 32 at a time, one a lane: phase 1 tests each against every home with the
+// FP32 squared distance alone and appends the accepted j to the home's queue (one ballot a home);
+// phase 2 takes a home's next 32 queued partners, one a lane, and evaluates every term. Within the
+// cutoffs of a dense system lie a few per cent of the particles, so evaluating in place would
+// run the pair body for one or two lanes of the warp in most windows; through the queue it runs
+// with all lanes busy, and the test, some 15 instructions for 32 pairs, is what bounds the kernel.
+// `split` warps (1, 2, 4 or 8) share a group of homes, each taking every split-th window, so that
+// small systems still fill the chip; the host picks it from n. The sums of the lanes and then
+// of the split warps are added in a fixed order.
+// Measured (pack and forces, us): one thread a particle in 64-thread blocks 139 / 798 / 2,285 at 500 /
+// 4,001 / 16,384 particles (63 blocks of 2 warps on 152 SMs at 4,001), this form 17 / 48 / 261. The
+// lanes' sums wait in shared memory: held in registers for four homes they took 118 of them, and
+// 16 warps an SM left 56% of the issue slots without a ready warp.
+// The pair terms of one home and one partner (steric.hpp, electrostatic.hpp, hydrophobic.hpp).
+__device__ __forceinline__ void na_pair(const NaParams &p, float4 pi, float4 qi, float4 pj, float4 qj, float (&v)[6])
+{
+    float &fx = v[0], &fy = v[1], &fz = v[2], &es = v[3], &ec = v[4], &eh = v[5];
+    const unsigned int fi = __float_as_uint(qi.w), fj = __float_as_uint(qj.w);
+    const float w = (fj & PF_STATIC) ? 1.0f : 0.5f;
+    const float dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
+    const float r2 = dx * dx + dy * dy + dz * dz;
+    float f = 0.0f;
+    if (p.steric_on && na_in(r2, p.lo2_s, p.hi2_s, pi, pj, p.c_steric, false))
+    {
+        float fod = 0.0f;
+        if (p.steric_mode == BS_STERIC_LINEAR)
+        {
+            // E = (d - (ri + rj))^2 / 2 when overlapping, |F| = |d - (ri + rj)|
+            const float d = sqrtf(r2);
+            const float dv = d - (pi.w + pj.w);
+            if (dv <= 0.0f)
+            {
+                fod = d > 0.0f ? dv / d : 0.0f;
+                es = fmaf(w * 0.5f, dv * dv, es);
+            }
+        }
+        else if (r2 >= 0.01f) // d < 0.1 A gives zero
+        {
+            const float inv2 = 1.0f / r2;
+            const float i6 = inv2 * inv2 * inv2;
+            const float t6 = pi.w * pj.w * i6;
+            if (p.steric_mode == BS_STERIC_LJ_12_6_AMBER)
+            {
+                const float t12 = qi.x * qj.x * i6 * i6;
+                es = fmaf(w, t12 - 2.0f * t6, es);
+                fod = 12.0f * (t6 - t12) * inv2;
+            }
+            else if (p.steric_mode == BS_STERIC_LJ_8_6_LEWITT)
+            {
+                const float t8 = qi.x * qj.x * i6 * inv2;
+                es = fmaf(w, 3.0f * t8 - 4.0f * t6, es);
+                fod = 24.0f * (t6 - t8) * inv2;
+            }
+            else
+            {
+                const float t8 = qi.x * qj.x * i6 * inv2;
+                es = fmaf(w, t8 - t6, es);
+                fod = (6.0f * t6 - 8.0f * t8) * inv2;
+            }
+        }
+        f = fod * p.kf_steric;
+    }
+    if (p.coulomb_on && (fi & fj & PF_CHARGED) && r2 >= 1e-6f &&
+        na_in(r2, p.lo2_c, p.hi2_c, pi, pj, p.c_coulomb, true))
+    {
+        const float inv = 1.0f / sqrtf(r2);
+        float tq = qi.y * qj.y * inv;
+        float fod;
+        if (p.dist_dielectric)
+        {
+            tq *= inv;
+            fod = -2.0f * tq * inv * inv;
+        }
+        else
+            fod = -tq * inv * inv;
+        ec = fmaf(w, tq, ec);
+        f = fmaf(fod, p.kf_elec, f);
+    }
+    if (p.hydro_on && (fi & fj & PF_HYDROPHOBIC) && na_in(r2, p.lo2_h, p.hi2_h, pi, pj, p.c_hydro, true))
+    {
+        const float d = sqrtf(r2);
+        const float x = qi.z * qj.z * expf(-d);
+        eh = fmaf(-w, x, eh);
+        f = fmaf(x / d, p.kf_hydro, f);
+    }
+    fx = fmaf(dx, f, fx);
+    fy = fmaf(dy, f, fy);
+    fz = fmaf(dz, f, fz);
+}
+
+__global__ void __launch_bounds__(kNaBlock, 3) k_na_forces(NaParams p, int split, float *__restrict__ forces,
                                                         double *__restrict__ energies, NaBuffers b)
 {
-    __shared__ float4 sh_pos[kNaBlock];
-    __shared__ float4 sh_prm[kNaBlock];
-    __shared__ double sh_e[kNaBlock / 32][kNaTerms];
+    constexpr int R = kNaHomes, W = kNaBlock / 32;
+    constexpr int NV = 6; // force x, y, z and three energies of a home
+    __shared__ unsigned short sh_queue[W][R][64];
+    __shared__ float4 sh_home[W][R];
+    __shared__ float sh_acc[W][R][NV][32]; // each lane's sums, out of the registers of phase 1
+    __shared__ float sh_sum[W][R][NV];
+    __shared__ double sh_e[W][kNaTerms];
     __shared__ bool last;
-    const int i = blockIdx.x * kNaBlock + threadIdx.x;
-    const bool valid = i < p.n;
-    const float4 pi = valid ? b.pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 qi = valid ? b.prm[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const unsigned int fi = __float_as_uint(qi.w);
-    const bool dyn = valid && !(fi & PF_STATIC);
-    const bool do_s = dyn && p.steric_on;
-    const bool do_c = dyn && p.coulomb_on && (fi & PF_CHARGED);
-    const bool do_h = dyn && p.hydro_on && (fi & PF_HYDROPHOBIC);
-    float sx = 0.f, sy = 0.f, sz = 0.f, es = 0.f; // steric
-    float cx = 0.f, cy = 0.f, cz = 0.f, ec = 0.f; // Coulomb
-    float hx = 0.f, hy = 0.f, hz = 0.f, eh = 0.f; // hydrophobic
-    for (int t0 = 0; t0 < p.n; t0 += kNaBlock)
-    {
-        const int jl = t0 + threadIdx.x;
-        __syncthreads();
-        if (jl < p.n)
-        {
-            sh_pos[threadIdx.x] = b.pos[jl];
-            sh_prm[threadIdx.x] = b.prm[jl];
-        }
-        __syncthreads();
-        const int m = min(kNaBlock, p.n - t0);
-        if (!(do_s || do_c || do_h))
-            continue;
-        for (int k = 0; k < m; ++k)
-        {
-            const int j = t0 + k;
-            if (j == i)
-                continue;
-            const float4 pj = sh_pos[k];
-            const float4 qj = sh_prm[k];
-            const unsigned int fj = __float_as_uint(qj.w);
-            const float w = (fj & PF_STATIC) ? 1.0f : 0.5f;
-            const float dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
-            const float r2 = dx * dx + dy * dy + dz * dz;
-            if (do_s && na_in(r2, p.lo2_s, p.hi2_s, pi, pj, p.c_steric, false))
-            {
-                if (p.steric_mode == BS_STERIC_LINEAR)
-                {
-                    // E = (d - (ri + rj))^2 / 2 when overlapping, |F| = |d - (ri + rj)|
-                    const float d = sqrtf(r2);
-                    const float dv = d - (pi.w + pj.w);
-                    if (dv <= 0.0f)
-                    {
-                        const float fod = d > 0.0f ? dv / d : 0.0f;
-                        es = fmaf(w * 0.5f, dv * dv, es);
-                        sx = fmaf(dx, fod, sx);
-                        sy = fmaf(dy, fod, sy);
-                        sz = fmaf(dz, fod, sz);
-                    }
-                }
-                else if (r2 >= 0.01f) // d < 0.1 A gives zero
-                {
-                    const float inv2 = 1.0f / r2;
-                    const float i6 = inv2 * inv2 * inv2;
-                    const float t6 = pi.w * pj.w * i6;
-                    float fod;
-                    if (p.steric_mode == BS_STERIC_LJ_12_6_AMBER)
-                    {
-                        const float t12 = qi.x * qj.x * i6 * i6;
-                        es = fmaf(w, t12 - 2.0f * t6, es);
-                        fod = 12.0f * (t6 - t12) * inv2;
-                    }
-                    else if (p.steric_mode == BS_STERIC_LJ_8_6_LEWITT)
-                    {
-                        const float t8 = qi.x * qj.x * i6 * inv2;
-                        es = fmaf(w, 3.0f * t8 - 4.0f * t6, es);
-                        fod = 24.0f * (t6 - t8) * inv2;
-                    }
-                    else
-                    {
-                        const float t8 = qi.x * qj.x * i6 * inv2;
-                        es = fmaf(w, t8 - t6, es);
-                        fod = (6.0f * t6 - 8.0f * t8) * inv2;
-                    }
-                    sx = fmaf(dx, fod, sx);
-                    sy = fmaf(dy, fod, sy);
-                    sz = fmaf(dz, fod, sz);
-                }
-            }
-            if (do_c && (fj & PF_CHARGED) && r2 >= 1e-6f && na_in(r2, p.lo2_c, p.hi2_c, pi, pj, p.c_coulomb, true))
-            {
-                const float inv = 1.0f / sqrtf(r2);
-                float tq = qi.y * qj.y * inv;
-                float fod;
-                if (p.dist_dielectric)
-                {
-                    tq *= inv;
-                    fod = -2.0f * tq * inv * inv;
-                }
-                else
-                    fod = -tq * inv * inv;
-                ec = fmaf(w, tq, ec);
-                cx = fmaf(dx, fod, cx);
-                cy = fmaf(dy, fod, cy);
-                cz = fmaf(dz, fod, cz);
-            }
-            if (do_h && (fj & PF_HYDROPHOBIC) && na_in(r2, p.lo2_h, p.hi2_h, pi, pj, p.c_hydro, true))
-            {
-                const float d = sqrtf(r2);
-                const float x = qi.z * qj.z * expf(-d);
-                const float fod = x / d;
-                eh = fmaf(-w, x, eh);
-                hx = fmaf(dx, fod, hx);
-                hy = fmaf(dy, fod, hy);
-                hz = fmaf(dz, fod, hz);
-            }
-        }
-    }
-    if (valid)
-    {
-        float fx = 0.f, fy = 0.f, fz = 0.f;
-        if (dyn)
-        {
-            fx = sx * p.kf_steric + cx * p.kf_elec + hx * p.kf_hydro;
-            fy = sy * p.kf_steric + cy * p.kf_elec + hy * p.kf_hydro;
-            fz = sz * p.kf_steric + cz * p.kf_elec + hz * p.kf_hydro;
-        }
-        forces[3 * i] = fx;
-        forces[3 * i + 1] = fy;
-        forces[3 * i + 2] = fz;
-    }
-    // ---- energies: warp sums in FP32, block and grid sums in FP64, fixed order ----
-    float e[kNaTerms] = {es * p.ke_steric, ec * p.ke_elec, eh * p.ke_hydro};
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    asm volatile("griddepcontrol.wait;" ::: "memory"); // the packed particles of k_na_pack
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int group = warp / split, part = warp % split; // home group in the block, share of its windows
+    const int h0 = (blockIdx.x * (W / split) + group) * R;
+    const unsigned int below = (1u << lane) - 1u;
+    float hx[R], hy[R], hz[R];
+    float r2max[R]; // 0: the home takes no pairs (static, past the end, or no term acts on it)
+    bool any = false;
 #pragma unroll
-    for (int q = 0; q < kNaTerms; ++q)
+    for (int r = 0; r < R; ++r)
     {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            e[q] += __shfl_down_sync(0xffffffffu, e[q], o);
+        const int i = h0 + r;
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        r2max[r] = 0.0f;
+        if (i < p.n)
+        {
+            x = b.pos[i];
+            const unsigned int fi = __float_as_uint(b.prm[i].w);
+            if (!(fi & PF_STATIC))
+            {
+                float m = p.steric_on ? p.hi2_s : 0.0f;
+                if (p.coulomb_on && (fi & PF_CHARGED))
+                    m = fmaxf(m, p.hi2_c);
+                if (p.hydro_on && (fi & PF_HYDROPHOBIC))
+                    m = fmaxf(m, p.hi2_h);
+                r2max[r] = m;
+            }
+        }
+        hx[r] = x.x;
+        hy[r] = x.y;
+        hz[r] = x.z;
         if (lane == 0)
-            sh_e[wid][q] = static_cast<double>(e[q]);
+            sh_home[warp][r] = x;
+#pragma unroll
+        for (int q = 0; q < NV; ++q)
+            sh_acc[warp][r][q][lane] = 0.0f;
+        any = any || r2max[r] > 0.0f;
+    }
+    // queued partners of each home (low half) and the place of the first in its ring of 64 (high half)
+    unsigned int fill[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+        fill[r] = 0u;
+    // up to 32 queued partners of home r, one a lane; r is the same in every lane but no constant, so
+    // that one copy of the pair body serves every home
+    auto evaluate = [&](int r, int first, int m) {
+        __syncwarp();
+        const int i = h0 + r;
+        const int j = lane < m ? sh_queue[warp][r][(first + lane) & 63] : i;
+        if (j != i)
+        {
+            float v[NV];
+#pragma unroll
+            for (int q = 0; q < NV; ++q)
+                v[q] = sh_acc[warp][r][q][lane];
+            na_pair(p, sh_home[warp][r], b.prm[i], b.pos[j], b.prm[j], v);
+#pragma unroll
+            for (int q = 0; q < NV; ++q)
+                sh_acc[warp][r][q][lane] = v[q];
+        }
+        __syncwarp(); // the slots may be filled again
+    };
+    if (any)
+    {
+        const float nan = __int_as_float(0x7fffffff); // past the end: no distance compares
+        const int step = 32 * split;
+        int k = 32 * part + lane;
+        float4 next = k < p.n ? b.pos[k] : make_float4(nan, nan, nan, 0.f);
+        for (int k0 = 32 * part; k0 < p.n; k0 += step)
+        {
+            const float4 pj = next;
+            const int j = k;
+            k += step;
+            next = k < p.n ? b.pos[k] : make_float4(nan, nan, nan, 0.f);
+            unsigned int full = 0u;
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+            {
+                const float dx = pj.x - hx[r], dy = pj.y - hy[r], dz = pj.z - hz[r];
+                const float r2 = dx * dx + dy * dy + dz * dz;
+                const bool in = r2 < r2max[r];
+                const unsigned int m = __ballot_sync(0xffffffffu, in);
+                if (in)
+                    sh_queue[warp][r][((fill[r] >> 16) + fill[r] + __popc(m & below)) & 63] = static_cast<unsigned short>(j);
+                fill[r] += __popc(m);
+                full |= (fill[r] & 0x20u) << r; // 32 or more queued (at most 63)
+            }
+            if (full)
+            {
+#pragma unroll 1
+                for (int r = 0; r < R; ++r)
+                {
+                    if (!((full >> r) & 0x20u))
+                        continue;
+                    unsigned int first = 0u;
+#pragma unroll
+                    for (int q = 0; q < R; ++q)
+                        if (q == r)
+                        {
+                            first = fill[q] >> 16;
+                            fill[q] += (32u << 16) - 32u;
+                        }
+                    evaluate(r, first, 32);
+                }
+            }
+        }
+#pragma unroll 1
+        for (int r = 0; r < R; ++r)
+        {
+            unsigned int f = 0u;
+#pragma unroll
+            for (int q = 0; q < R; ++q)
+                f = q == r ? fill[q] : f;
+            if (f & 0xffffu)
+                evaluate(r, f >> 16, f & 0xffffu);
+        }
+    }
+#pragma unroll 1
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int q = 0; q < NV; ++q)
+        {
+            float v = sh_acc[warp][r][q][lane];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                v += __shfl_down_sync(0xffffffffu, v, o);
+            if (lane == 0)
+                sh_sum[warp][r][q] = v;
+        }
+    __syncthreads();
+    // one thread a home adds the split warps' sums; energies go on in FP64, home by home
+    if (part == 0 && lane < R)
+    {
+        float v[NV] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        for (int s = 0; s < split; ++s)
+#pragma unroll
+            for (int q = 0; q < NV; ++q)
+                v[q] += sh_sum[warp + s][lane][q];
+        const int i = h0 + lane;
+        if (i < p.n)
+        {
+            forces[3 * i] = v[0];
+            forces[3 * i + 1] = v[1];
+            forces[3 * i + 2] = v[2];
+        }
+        double e[kNaTerms] = {static_cast<double>(v[3]) * p.ke_steric, static_cast<double>(v[4]) * p.ke_elec,
+                              static_cast<double>(v[5]) * p.ke_hydro};
+#pragma unroll
+        for (int q = 0; q < kNaTerms; ++q)
+        {
+#pragma unroll
+            for (int o = R / 2; o > 0; o >>= 1)
+                e[q] += __shfl_down_sync((1u << R) - 1u, e[q], o, R);
+            if (lane == 0)
+                sh_e[group][q] = e[q];
+        }
     }
     __syncthreads();
     if (threadIdx.x == 0)
@@ -308,29 +428,56 @@ __global__ void __launch_bounds__(kNaBlock) k_na_forces(NaParams p, float *__res
         for (int q = 0; q < kNaTerms; ++q)
         {
             double s = 0.0;
-            for (int w = 0; w < kNaBlock / 32; ++w)
-                s += sh_e[w][q];
+            for (int g = 0; g < W / split; ++g)
+                s += sh_e[g][q];
             b.blk[blockIdx.x * kNaTerms + q] = s;
         }
         __threadfence();
         last = atomicAdd(b.done, 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    if (!last || threadIdx.x != 0)
+    if (!last)
         return;
+    // the last block adds the blocks' energies: thread t takes blocks t, t + 256, ... in order, then
+    // a fixed tree
     __threadfence();
     double tot[kNaTerms] = {0.0, 0.0, 0.0};
-    for (unsigned int k = 0; k < gridDim.x; ++k)
+    for (unsigned int k = threadIdx.x; k < gridDim.x; k += kNaBlock)
 #pragma unroll
         for (int q = 0; q < kNaTerms; ++q)
-            tot[q] += *(volatile double *)&b.blk[k * kNaTerms + q];
-    for (int q = 0; q < BS_NUM_ENERGIES; ++q)
-        energies[q] = 0.0;
-    energies[BS_ENERGY_STERIC] = tot[0];
-    energies[BS_ENERGY_ELECTROSTATIC] = tot[1];
-    energies[BS_ENERGY_HYDROPHOBIC] = tot[2];
-    *b.done = 0u; // ready for the next call
+            tot[q] += __ldcg(&b.blk[k * kNaTerms + q]);
+#pragma unroll
+    for (int q = 0; q < kNaTerms; ++q)
+    {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            tot[q] += __shfl_down_sync(0xffffffffu, tot[q], o);
+        if (lane == 0)
+            sh_e[warp][q] = tot[q];
+    }
+    __syncthreads();
+    if (threadIdx.x < BS_NUM_ENERGIES)
+    {
+        const int q = threadIdx.x == BS_ENERGY_STERIC          ? 0
+                      : threadIdx.x == BS_ENERGY_ELECTROSTATIC ? 1
+                      : threadIdx.x == BS_ENERGY_HYDROPHOBIC   ? 2
+                                                               : -1;
+        double s = 0.0;
+        if (q >= 0)
+            for (int w = 0; w < W; ++w)
+                s += sh_e[w][q];
+        energies[threadIdx.x] = s;
+    }
+    if (threadIdx.x == 0)
+        *b.done = 0u; // ready for the next call
 }
+
+// Warps that share a group of homes: some 8,000 warps up to 10,000 particles (four times what the
+// chip holds at once), so that the last blocks to finish are short; half as many homes a block cost
+// more in part-filled queues than they gain. Measured (us a call, 2,500 / 5,000 / 10,000 / 16,384
+// particles): this rule 31 / 56 / 124 / 261; a warp for every group from 10,000 and half the split
+// below 31 / 54 / 129 / 307; the split halved again 29 / 57 / 156 / 307.
+int na_split(int n) { return n <= 5000 ? 8 : (n <= 10000 ? 4 : 2); }
 
 float na_band_lo2(double c) { return static_cast<float>((c * (1.0 - 1.0 / 16384.0)) * (c * (1.0 - 1.0 / 16384.0))); }
 float na_band_hi2(double c) { return static_cast<float>((c * (1.0 + 1.0 / 16384.0)) * (c * (1.0 + 1.0 / 16384.0))); }
@@ -475,7 +622,18 @@ extern "C" int bs_nonbonded_forces_noalloc(const bs_config *cfg, int64_t n, cons
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     k_na_pack<<<(p.n + 255) / 256, 256, 0, st>>>(p, d_xyz, d_radius, d_epsilon, d_charge, d_hydrophobicity,
                                                   d_is_static, b);
-    k_na_forces<<<(p.n + kNaBlock - 1) / kNaBlock, kNaBlock, 0, st>>>(p, d_forces, d_energies, b);
+    // the force kernel starts launching while the packing runs and waits for it on the device
+    const int split = na_split(p.n), per_block = kNaHomes * (kNaMaxSplit / split);
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3((p.n + per_block - 1) / per_block);
+    lc.blockDim = dim3(kNaBlock);
+    lc.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = attr;
+    lc.numAttrs = 1;
+    cudaLaunchKernelEx(&lc, k_na_forces, p, split, d_forces, d_energies, b);
     rc = cudaGetLastError();
     if (rc != cudaSuccess)
     {
