@@ -308,6 +308,8 @@ int rebuild_now(bs_sim *s)
         const int st = s->ctl_host->status;
         if (st & ST_NONFINITE)
             return fail(s, BS_E_NONFINITE, "non-finite particle position");
+        if (st & ST_BARRIER)
+            return fail(s, BS_E_CUDA, "a grid barrier of the step kernel timed out");
         if (st & ST_CELL_CAPACITY)
         {
             const long long need = s->ctl_host->ncells_needed;
@@ -367,8 +369,7 @@ int capture_period_graph(bs_sim *s)
     cudaGraph_t g = nullptr;
     BS_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
     int kernels = launch_rebuild(s->p, s->stream);
-    for (int k = 0; k < K; ++k)
-        kernels += launch_step(s->p, MODE_STEP, s->stream);
+    kernels += launch_steps(s->p, K, s->stream);
     BS_CUDA(cudaStreamEndCapture(s->stream, &g));
     const cudaError_t e = cudaGraphInstantiate(&s->period_graph, g, 0);
     cudaGraphDestroy(g);
@@ -1476,6 +1477,16 @@ int bs_setup(bs_sim *s, const bs_config *cfg)
     p.k_imp_f = static_cast<float>(kImpForceConvert);
     p.k_hydro_e = static_cast<float>(kAvogadro * 1.0E-3);
 
+    bool fits = false;
+    BS_CUDA(run_fits(p, &fits));
+    if (fits)
+    {
+        BS_CUDA(s->dev.alloc(&p.run_arrive, 1));
+        BS_CUDA(cudaMemsetAsync(p.run_arrive, 0, sizeof(unsigned int), s->stream));
+        BS_CUDA(s->dev.alloc(&p.run_probe, 16 * static_cast<size_t>(run_blocks(p))));
+        p.run_on = 1;
+    }
+
     s->ready = true;
     s->steps_done = 0;
     s->target = 0;
@@ -1528,8 +1539,7 @@ static int enqueue_steps(bs_sim *s, long long count)
             s->since_rebuild = 0;
         }
         const long long chunk = std::min<long long>(remaining, K - s->since_rebuild);
-        for (long long k = 0; k < chunk; ++k)
-            s->launches += launch_step(s->p, MODE_STEP, s->stream);
+        s->launches += launch_steps(s->p, static_cast<int>(chunk), s->stream);
         s->since_rebuild += static_cast<int>(chunk);
         remaining -= chunk;
     }
@@ -1617,6 +1627,8 @@ int bs_synchronize(bs_sim *s)
         s->steps_done = h.steps;
         if (h.status & ST_NONFINITE)
             return fail(s, BS_E_NONFINITE, "Found non-finite position (a particle position became NaN or infinite)");
+        if (h.status & ST_BARRIER)
+            return fail(s, BS_E_CUDA, "a grid barrier of the step kernel timed out");
         if (h.status & (ST_CELL_CAPACITY | ST_PAIR_CAPACITY | ST_WIDE))
         {
             rc = rebuild_now(s); // grows the lists and rebuilds

@@ -40,6 +40,7 @@ enum : int
     ST_CELL_CAPACITY = 4,   // the search grid needs more cells than allocated
     ST_STALE = 8,           // a particle drifted more than half the list skin: rebuild needed
     ST_WIDE = 16,           // a neighbour offset does not fit the 16-bit steric list
+    ST_BARRIER = 32,        // a grid barrier's bounded wait ran out
 };
 
 // particle flag bits
@@ -202,6 +203,10 @@ struct Params
     double *blk_energy;       // block and group partials of the step energies, group counters
     int blk_cap;              // block partials it holds (the step kernel's largest grid)
     Ctl *ctl;
+    // kernels of several steps (bs_run.cu)
+    int run_on;               // the system's step grid is resident at once: k_run takes its steps
+    unsigned int *run_arrive; // grid-barrier word, 0 between launches
+    float *run_probe;         // [2][blocks][8] the probe's per-block sums, by the parity of the step
     // configuration
     float dt;
     int spring_on, steric_on, coulomb_on, hydro_on, imp_on, visc_on;

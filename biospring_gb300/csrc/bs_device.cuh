@@ -29,6 +29,25 @@ __device__ __forceinline__ void pdl_enter()
 #endif
 }
 
+// Positions as the force loops read them. PosConst: written by an earlier kernel only, read through
+// the non-coherent path. PosShared: written by other blocks of the same kernel between its barriers
+// (kernels that run several steps), read with ordinary loads, which a barrier's acquire orders.
+struct PosConst
+{
+    const float4 *__restrict__ p;
+    __device__ __forceinline__ float4 operator[](int j) const { return __ldg(p + j); }
+};
+struct PosShared
+{
+    const float4 *p;
+    __device__ __forceinline__ float4 operator[](int j) const
+    {
+        float4 v;
+        asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p + j));
+        return v;
+    }
+};
+
 __device__ __forceinline__ unsigned int f2ord(float f)
 {
     const unsigned int b = __float_as_uint(f);
@@ -289,11 +308,50 @@ __device__ __forceinline__ bool reduce_energies(const float (&e)[NE], double *bl
     return true;
 }
 
+// The step energies, reduced in the order spring, steric, Coulomb, hydrophobic, IMPALA, kinetic, to their
+// BS_ENERGY_* places. One thread.
+__device__ __forceinline__ void publish_energies(Ctl *ctl)
+{
+    const double sp = ctl->energies[0], st = ctl->energies[1], co = ctl->energies[2], hy = ctl->energies[3],
+                 im = ctl->energies[4], ki = ctl->energies[5];
+    ctl->energies[BS_ENERGY_KINETIC] = ki;
+    ctl->energies[BS_ENERGY_SPRING] = sp;
+    ctl->energies[BS_ENERGY_STERIC] = st;
+    ctl->energies[BS_ENERGY_ELECTROSTATIC] = co;
+    ctl->energies[BS_ENERGY_IMP] = im;
+    ctl->energies[BS_ENERGY_HYDROPHOBIC] = hy;
+}
+
+// The probe's step under the force F of the particles (SpringNetwork.cpp:156-182): viscosity from its
+// velocity, the Euler step (Particle.cpp:109-128) and its kinetic energy.
+__device__ __forceinline__ void probe_advance(const Params &p, float *F, float4 &x, float4 &v, float &ke)
+{
+    if (p.visc_on)
+    {
+        F[0] = __fsub_rn(F[0], __fmul_rn(v.x, p.visc));
+        F[1] = __fsub_rn(F[1], __fmul_rn(v.y, p.visc));
+        F[2] = __fsub_rn(F[2], __fmul_rn(v.z, p.visc));
+    }
+    const float m = p.probe_mass;
+    if (m > 0.0f)
+    {
+        v.x = __fadd_rn(v.x, __fmul_rn(__fdiv_rn(F[0], m), p.dt));
+        v.y = __fadd_rn(v.y, __fmul_rn(__fdiv_rn(F[1], m), p.dt));
+        v.z = __fadd_rn(v.z, __fmul_rn(__fdiv_rn(F[2], m), p.dt));
+    }
+    const double vx = v.x, vy = v.y, vz = v.z;
+    const float vit = static_cast<float>(sqrt(__dadd_rn(__dadd_rn(__dmul_rn(vx, vx), __dmul_rn(vy, vy)), __dmul_rn(vz, vz))));
+    ke = 0.5f * m * (vit * vit) * p.k_kin;
+    x.x = __fadd_rn(x.x, __fmul_rn(v.x, p.dt));
+    x.y = __fadd_rn(x.y, __fmul_rn(v.y, p.dt));
+    x.z = __fadd_rn(x.z, __fmul_rn(v.z, p.dt));
+}
+
 // Springs of slot s handled by lane t of T (Spring.cpp:20-34, spring.hpp:17-29). Returns the
 // force before the unit conversion and scale, and the weighted energy before the scale.
-template <int T>
+template <int T, class POS>
 __device__ __forceinline__ void spring_forces(const Params &p, int s, int t, float4 pi,
-                                              const float4 *__restrict__ pos, float &fx, float &fy, float &fz,
+                                              const POS pos, float &fx, float &fy, float &fz,
                                               float &e)
 {
     const int deg = p.se_deg[s];
@@ -306,7 +364,7 @@ __device__ __forceinline__ void spring_forces(const Params &p, int s, int t, flo
     float kn = __ldg(&p.se_k[at]), rn = __ldg(&p.se_r0[at]);
     float4 pn = make_float4(0.f, 0.f, 0.f, 0.f);
     if (!(cn & kEntryInactive))
-        pn = __ldg(&pos[cn & kSlotMask]);
+        pn = pos[cn & kSlotMask];
     for (int k = t; k < deg; k += T)
     {
         const unsigned int c = cn;
@@ -319,7 +377,7 @@ __device__ __forceinline__ void spring_forces(const Params &p, int s, int t, flo
             kn = __ldg(&p.se_k[at]);
             rn = __ldg(&p.se_r0[at]);
             if (!(cn & kEntryInactive))
-                pn = __ldg(&pos[cn & kSlotMask]);
+                pn = pos[cn & kSlotMask];
         }
         if (c & kEntryInactive)
             continue;
@@ -342,9 +400,9 @@ __device__ __forceinline__ void spring_forces(const Params &p, int s, int t, flo
 // energy); KIND 1: list 0 in 32-bit mode; KIND 2: list 3 (static partners, full energy).
 // The loop is software-pipelined: entries are loaded two iterations ahead of use and
 // positions (and the LJ factor of the partner) one iteration ahead.
-template <int SM, int T, int KIND>
+template <int SM, int T, int KIND, class POS>
 __device__ __forceinline__ void steric_forces(const Params &p, int s, int t, float4 pi, float fhi_i,
-                                              const float4 *__restrict__ pos, const float *__restrict__ fhi,
+                                              const POS pos, const float *__restrict__ fhi,
                                               float &fx, float &fy, float &fz, float &e)
 {
     const PairList &L = p.pl[KIND == 2 ? kListStericStatic : 0];
@@ -364,7 +422,7 @@ __device__ __forceinline__ void steric_forces(const Params &p, int s, int t, flo
     constexpr bool LJ = SM != BS_STERIC_LINEAR;
     int jn = entry(t);
     int jn2 = t + T < cnt ? entry(t + T) : 0;
-    float4 pn = __ldg(&pos[jn]);
+    float4 pn = pos[jn];
     float hn = LJ ? __ldg(&fhi[jn]) : 0.0f;
     for (int k = t; k < cnt; k += T)
     {
@@ -375,7 +433,7 @@ __device__ __forceinline__ void steric_forces(const Params &p, int s, int t, flo
             jn2 = entry(k + 2 * T);
         if (k + T < cnt)
         {
-            pn = __ldg(&pos[jn]);
+            pn = pos[jn];
             if (LJ)
                 hn = __ldg(&fhi[jn]);
         }
@@ -481,9 +539,9 @@ __device__ __forceinline__ float lj_pair(float r2, bool ok, float pw, float fhi_
 // warp waits for one round trip per U pairs instead of one per pair. Entries past the row's end
 // read the slot past the particles (far from all of them) and fail the distance test. Rows start on 16-byte boundaries (capacities are
 // multiples of 8 entries), so the vector loads are aligned and never leave the row's capacity.
-template <int SM, int T, bool PL16, bool UF = false>
+template <int SM, int T, bool PL16, bool UF, class POS>
 __device__ __forceinline__ void steric_forces_batched(const Params &p, int s, int t, float4 pi, float fhi_i,
-                                                      const float4 *__restrict__ pos, const float *__restrict__ fhi,
+                                                      const POS pos, const float *__restrict__ fhi,
                                                       float &fx, float &fy, float &fz, float &e, int cnt_in = -1,
                                                       uint2 w16_in = make_uint2(0u, 0u))
 {
@@ -575,7 +633,7 @@ __device__ __forceinline__ void steric_forces_batched(const Params &p, int s, in
             // is read instead, and its squared distance (infinite) rejects it below
             if ((BS_GATHER == 2 ? base + T * u : base + u) >= cnt)
                 j[u] = p.npad;
-            pj[u] = __ldg(&pos[j[u]]);
+            pj[u] = pos[j[u]];
             hj[u] = LJ ? (UF ? p.lj_F : __ldg(&fhi[j[u]])) : 0.0f; // one LJ type: no factor to gather
         }
         unsigned int band = 0u; // LJ pairs of this pass within the guard band (BS_LJ_BAND_AFTER)
@@ -644,9 +702,9 @@ __device__ __forceinline__ void steric_forces_batched(const Params &p, int s, in
 // Springs of slot s, lane t of T, in passes of kGatherU entries per lane (entries t + T u of the
 // ELL row, the same entries in the same order as spring_forces): the U entries' columns are read
 // first, then the U partner positions together.
-template <int T>
+template <int T, class POS>
 __device__ __forceinline__ void spring_forces_batched(const Params &p, int s, int t, float4 pi,
-                                                      const float4 *__restrict__ pos, float &fx, float &fy, float &fz,
+                                                      const POS pos, float &fx, float &fy, float &fz,
                                                       float &e)
 {
     constexpr int U = kGatherU;
@@ -674,7 +732,7 @@ __device__ __forceinline__ void spring_forces_batched(const Params &p, int s, in
         }
 #pragma unroll
         for (int u = 0; u < U; ++u)
-            pj[u] = (c[u] & kEntryInactive) ? pi : __ldg(&pos[c[u] & kSlotMask]);
+            pj[u] = (c[u] & kEntryInactive) ? pi : pos[c[u] & kSlotMask];
 #pragma unroll
         for (int u = 0; u < U; ++u)
         {
@@ -697,9 +755,9 @@ __device__ __forceinline__ void spring_forces_batched(const Params &p, int s, in
 
 // Coulomb pairs of a charged slot, lane t of T (Particle.cpp:191-253, electrostatic.hpp:16-49).
 // With the distance-dependent dielectric eps = D r, E = K q q / (D r^2) and F = -dE/dr.
-template <int T>
+template <int T, class POS>
 __device__ __forceinline__ void coulomb_forces(const Params &p, int s, int t, float4 pi, float qi,
-                                               const float4 *__restrict__ pos, const float *__restrict__ chg,
+                                               const POS pos, const float *__restrict__ chg,
                                                float &fx, float &fy, float &fz, float &e)
 {
     const PairList &L = p.pl[1];
@@ -711,7 +769,7 @@ __device__ __forceinline__ void coulomb_forces(const Params &p, int s, int t, fl
     // software-pipelined like the steric loop: entries two ahead, partner data one ahead
     unsigned int jn = __ldg(row + t);
     unsigned int jn2 = t + T < cnt ? __ldg(row + t + T) : 0u;
-    float4 pn = __ldg(&pos[jn & kSlotMask]);
+    float4 pn = pos[jn & kSlotMask];
     float qn = __ldg(&chg[jn & kSlotMask]);
     for (int k = t; k < cnt; k += T)
     {
@@ -723,7 +781,7 @@ __device__ __forceinline__ void coulomb_forces(const Params &p, int s, int t, fl
             jn2 = __ldg(row + k + 2 * T);
         if (k + T < cnt)
         {
-            pn = __ldg(&pos[jn & kSlotMask]);
+            pn = pos[jn & kSlotMask];
             qn = __ldg(&chg[jn & kSlotMask]);
         }
         const float dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
@@ -752,9 +810,9 @@ __device__ __forceinline__ void coulomb_forces(const Params &p, int s, int t, fl
 }
 
 // Hydrophobic pairs, lane t of T (Particle.cpp:269-330, hydrophobic.hpp:20-39).
-template <int T>
+template <int T, class POS>
 __device__ __forceinline__ void hydro_forces(const Params &p, int s, int t, float4 pi, float hi,
-                                             const float4 *__restrict__ pos, const float *__restrict__ hyd,
+                                             const POS pos, const float *__restrict__ hyd,
                                              float &fx, float &fy, float &fz, float &e)
 {
     const PairList &L = p.pl[2];
@@ -763,7 +821,7 @@ __device__ __forceinline__ void hydro_forces(const Params &p, int s, int t, floa
     for (int k = t; k < cnt; k += T)
     {
         const unsigned int j = __ldg(row + k);
-        const float4 pj = __ldg(&pos[j & kSlotMask]);
+        const float4 pj = pos[j & kSlotMask];
         const float dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
         const float r2 = dx * dx + dy * dy + dz * dz;
         if (!pair_in(r2, p.lo2_h, p.hi2_h, pi, pj, p.c_hydro, true))
@@ -975,11 +1033,12 @@ template <int T> __device__ __forceinline__ float group_sum(float v)
 // Coulomb rows walked by the whole warp. The batched kernel leaves both out (fewer live registers
 // under its 64-register budget: with them its spills grew and its step slowed by 7%); it walks
 // Coulomb rows with the particle's own lanes (the same pairs, summed in another order).
-template <int MODE, int SM, int T, bool SINGLE = true, bool LEAN = false>
+template <int MODE, int SM, int T, bool SINGLE = true, bool LEAN = false, class POS = PosConst>
 __device__ __forceinline__ int particle_step(const Params &p, const int s, const int t, const int send,
-                                             const int sb, const int lb, const bool ext_on, float (&eacc)[6])
+                                             const int sb, const int lb, const bool ext_on, const float4 *probe,
+                                             float (&eacc)[6])
 {
-    const float4 *__restrict__ pos = p.pos[sb];
+    const POS pos{p.pos[sb]};
     const bool lead = t == 0;
     int pend = 0;
 
@@ -1020,9 +1079,9 @@ __device__ __forceinline__ int particle_step(const Params &p, const int s, const
             else if ((SINGLE && BS_GATHER) || (!SINGLE && BS_GATHER_BATCH))
             {
                 if (p.pl16)
-                    steric_forces_batched<SM, T, true>(p, s, t, pi, fhi_i, pos, p.fhi[lb], sx, sy, sz, es);
+                    steric_forces_batched<SM, T, true, false>(p, s, t, pi, fhi_i, pos, p.fhi[lb], sx, sy, sz, es);
                 else
-                    steric_forces_batched<SM, T, false>(p, s, t, pi, fhi_i, pos, p.fhi[lb], sx, sy, sz, es);
+                    steric_forces_batched<SM, T, false, false>(p, s, t, pi, fhi_i, pos, p.fhi[lb], sx, sy, sz, es);
             }
             else if (p.pl16)
                 steric_forces<SM, T, 0>(p, s, t, pi, fhi_i, pos, p.fhi[lb], sx, sy, sz, es);
@@ -1181,7 +1240,7 @@ __device__ __forceinline__ int particle_step(const Params &p, const int s, const
             // ---- probe (SpringNetwork.cpp:156-182), after every other term ----
             if (!LEAN && p.probe_on)
             {
-                const float4 prb = p.ctl->probe_pos;
+                const float4 prb = *probe;
                 float px = 0.f, py = 0.f, pz = 0.f;
                 probe_pair<SM>(p, prb, pi, p.fhi[lb][s], p.chg[lb][s], px, py, pz, e[1], e[2]);
                 fx += px;

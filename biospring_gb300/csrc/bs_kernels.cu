@@ -886,22 +886,15 @@ __global__ void __launch_bounds__(kStepKernelBlock, kStepMinBlocks) k_step(Param
     const int sb = ctl->sbuf, lb = ctl->lbuf;
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     float e[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    const int pend = particle_step<MODE, SM, T, true, LEAN>(p, g / T, g % T, p.n, sb, lb, ctl->ext_pending != 0, e);
+    const int pend = particle_step<MODE, SM, T, true, LEAN>(p, g / T, g % T, p.n, sb, lb, ctl->ext_pending != 0,
+                                                               &ctl->probe_pos, e);
     if (pend)
         atomicOr(&ctl->status_pending, pend);
     if (reduce_energies<6, kStepKernelBlock>(e, p.blk_energy, p.blk_cap, &ctl->done_step, ctl->energies))
     {
         if (threadIdx.x == 0)
         {
-            // energies[] were written in e[] order: spring, steric, coulomb, hydrophobic, imp, kinetic
-            const double sp = ctl->energies[0], st = ctl->energies[1], co = ctl->energies[2],
-                         hy = ctl->energies[3], im = ctl->energies[4], ki = ctl->energies[5];
-            ctl->energies[BS_ENERGY_KINETIC] = ki;
-            ctl->energies[BS_ENERGY_SPRING] = sp;
-            ctl->energies[BS_ENERGY_STERIC] = st;
-            ctl->energies[BS_ENERGY_ELECTROSTATIC] = co;
-            ctl->energies[BS_ENERGY_IMP] = im;
-            ctl->energies[BS_ENERGY_HYDROPHOBIC] = hy;
+            publish_energies(ctl);
             if (MODE == MODE_STEP)
             {
                 ctl->sbuf = sb ^ 1;
@@ -966,25 +959,8 @@ __global__ void __launch_bounds__(1024) k_probe(Params p)
         F[k] = __fadd_rn(hi, lo);
     }
     float4 v = ctl->probe_vel, x = ctl->probe_pos;
-    if (p.visc_on)
-    {
-        F[0] = __fsub_rn(F[0], __fmul_rn(v.x, p.visc));
-        F[1] = __fsub_rn(F[1], __fmul_rn(v.y, p.visc));
-        F[2] = __fsub_rn(F[2], __fmul_rn(v.z, p.visc));
-    }
-    const float m = p.probe_mass;
-    if (m > 0.0f)
-    {
-        v.x = __fadd_rn(v.x, __fmul_rn(__fdiv_rn(F[0], m), p.dt));
-        v.y = __fadd_rn(v.y, __fmul_rn(__fdiv_rn(F[1], m), p.dt));
-        v.z = __fadd_rn(v.z, __fmul_rn(__fdiv_rn(F[2], m), p.dt));
-    }
-    const double vx = v.x, vy = v.y, vz = v.z;
-    const float vit = static_cast<float>(sqrt(__dadd_rn(__dadd_rn(__dmul_rn(vx, vx), __dmul_rn(vy, vy)), __dmul_rn(vz, vz))));
-    const float ke = 0.5f * m * (vit * vit) * p.k_kin;
-    x.x = __fadd_rn(x.x, __fmul_rn(v.x, p.dt));
-    x.y = __fadd_rn(x.y, __fmul_rn(v.y, p.dt));
-    x.z = __fadd_rn(x.z, __fmul_rn(v.z, p.dt));
+    float ke;
+    probe_advance(p, F, x, v, ke);
     ctl->probe_pos = x;
     ctl->probe_vel = v;
     ctl->energies[BS_ENERGY_KINETIC] += static_cast<double>(ke);
@@ -1257,14 +1233,6 @@ int launch_rebuild(const Params &p, cudaStream_t st)
     return launched + 1;
 }
 
-// The lean step kernel leaves out, at compile time, the terms most systems do not use (pairwise
-// hydrophobic forces, field grids, the probe, rigid bodies, float-float positions): fewer live
-// registers, so the common kernel runs without register spills.
-static bool lean_step(const Params &p)
-{
-    return BS_LEAN && !(p.hydro_on || p.fg_on[0] || p.fg_on[1] || p.probe_on || p.nbody > 0 || p.pos_lo[0]);
-}
-
 template <int MODE, int SM>
 static void launch_step_lanes(const Params &p, cudaStream_t st)
 {
@@ -1431,6 +1399,18 @@ int launch_step(const Params &p, int mode, cudaStream_t st)
         BS_STEP_LAUNCH(k_frame, std::min((p.n + 255) / 256, 608), 256, 0, st, p);
         launched += 2;
     }
+    return launched;
+}
+
+int launch_steps(const Params &p, int count, cudaStream_t st)
+{
+    int launched = 0;
+    if (p.run_on && p.frame_every == 0) // frames are recorded between two steps
+        for (int k = 0; k < count; k += kRunMaxSteps, ++launched)
+            launch_run(p, std::min(kRunMaxSteps, count - k), st);
+    else
+        for (int k = 0; k < count; ++k)
+            launched += launch_step(p, MODE_STEP, st);
     return launched;
 }
 

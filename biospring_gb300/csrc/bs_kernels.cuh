@@ -23,7 +23,7 @@ constexpr int kBboxBlock = 256;
 constexpr int kMaxEnergyBlocks = 1 << 16;
 
 // status bits that stop a rebuild; a stale list is what a rebuild repairs
-constexpr int kRebuildBlocking = ST_NONFINITE | ST_PAIR_CAPACITY | ST_CELL_CAPACITY | ST_WIDE;
+constexpr int kRebuildBlocking = ST_NONFINITE | ST_PAIR_CAPACITY | ST_CELL_CAPACITY | ST_WIDE | ST_BARRIER;
 // Programmatic dependent launch in the rebuild chain (its eleven kernels overlap their launches:
 // 351 -> 344 us at 100k). BS_PDL_STEP extends it to the step kernels, which made the graph-replayed
 // 100k step slower (120 -> 130 us), so it is off.
@@ -99,6 +99,23 @@ int launch_rebuild(const Params &p, cudaStream_t stream);
 int launch_step(const Params &p, int mode, cudaStream_t stream);      // step kernel, then the bodies
 int launch_step_only(const Params &p, int mode, cudaStream_t stream); // the step kernel alone
 int launch_rigid(const Params &p, cudaStream_t stream);               // bs_rigid.cu
+// count steps without a rebuild in between: one kernel where the system allows (Params::run_on)
+int launch_steps(const Params &p, int count, cudaStream_t stream);
+// bs_run.cu: the kernel of several steps, its blocks, and whether they are resident at once
+cudaError_t launch_run(const Params &p, int count, cudaStream_t stream);
+cudaError_t run_fits(const Params &p, bool *fits);
+int run_blocks(const Params &p);
+// Steps of one launch (10 in the default schedule) and the polls after which a barrier gives up (some
+// seconds; a meeting takes about a microsecond).
+constexpr int kRunMaxSteps = 1024;
+constexpr int kRunSpinLimit = 1 << 22;
+// The lean step kernels leave out, at compile time, the terms most systems do not use (pairwise
+// hydrophobic forces, field grids, the probe, rigid bodies, float-float positions): fewer live
+// registers, so the common kernel runs without register spills.
+inline bool lean_step(const Params &p)
+{
+    return BS_LEAN && !(p.hydro_on || p.fg_on[0] || p.fg_on[1] || p.probe_on || p.nbody > 0 || p.pos_lo[0]);
+}
 int launch_ext_add(const Params &p, long long i, float fx, float fy, float fz, cudaStream_t stream);
 int launch_set_burying(const Params &p, const float *burying, cudaStream_t stream);
 int launch_set_charges(const Params &p, const float *q, cudaStream_t st);

@@ -1,0 +1,262 @@
+// bs_run.cu -- several steps of one system in one kernel.
+//
+// A small system's step is latency, not work: a kernel a step pays the launch, the first reads of
+// the control block and the parameters, and the energy reduction (two device-wide fences and
+// counters in a row) for some 4 us of gathering. k_run is launched cooperatively, one thread group a
+// particle as in k_step, and takes all steps up to the next list rebuild: between two steps stands one
+// grid barrier (bodies take a second one), and the energies, which only the last step of a
+// call can show, are reduced once, by that step's own partials. The particle's step is particle_step
+// and the reduction reduce_energies, over the same blocks and in the same order as k_step's, so the
+// results are the same bit for bit. The probe's reaction is summed block by block, and every block then
+// computes the probe's step itself, so it costs no barrier of its own.
+//
+// Bound: the chain of dependent loads of a step, then the barrier. Measured, a call of 50 to 100 steps
+// with its rebuilds, a kernel a step against this one: Calpha network of 2,000 1,423 -> 905 us (100
+// steps), Lennard-Jones beads 5,003 431 -> 339 us (20), receptor and ligand of 6,007 with the probe 677 ->
+// 530 us (20), membrane of 20,000 with four bodies 1,460 -> 1,284 us (50).
+
+#include "bs_rigid.cuh"
+
+namespace bsg
+{
+namespace
+{
+
+static_assert(kRigidBlock == kStepKernelBlock, "k_run's blocks serve the bodies");
+
+// All blocks of the (cooperative) grid meet; gen counts the meetings of this launch from 1. Returns 1,
+// or 2 in every block alike if a thread of any block came with `pend` set, or 0 if this block gave the
+// (bounded) wait up: the others then do so too, and the launch ends without advancing the state.
+// Two flag bits, by the parity of gen: a block may already be at the next meeting when another reads
+// the word, but never two ahead.
+constexpr unsigned int kRunCount = (1u << 30) - 1u;
+__device__ __forceinline__ int grid_barrier(unsigned int *arrive, unsigned int gen, int pend)
+{
+    __shared__ int met;
+    const int any = __syncthreads_or(pend);
+    if (threadIdx.x == 0)
+    {
+        const unsigned int want = gen * gridDim.x, flag = 1u << (30 + (gen & 1u));
+        if (any)
+            atomicOr(arrive, flag);
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrive) : "memory");
+        unsigned int seen = 0;
+        int tries = 0;
+        do
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(arrive) : "memory");
+        while ((seen & kRunCount) < want && ++tries < kRunSpinLimit);
+        met = (seen & kRunCount) < want ? 0 : ((seen & flag) ? 2 : 1);
+    }
+    __syncthreads();
+    return met;
+}
+
+// The probe's sum over this block's particles, (hi, lo) per axis, into the block's row of `part`.
+__device__ __forceinline__ void probe_block_sum(const Params &p, const int first, const int count, float *part)
+{
+    // one warp an axis: 16 to 64 particles a block
+    const int lane = threadIdx.x & 31, axis = threadIdx.x >> 5;
+    __syncthreads();
+    if (axis >= 3)
+        return;
+    float hi = 0.0f, lo = 0.0f;
+    for (int s = first + lane; s < first + count; s += 32)
+        ff_add(hi, lo, reinterpret_cast<const float *>(p.probe_f + s)[axis], 0.0f);
+    warp_ff_sum(hi, lo);
+    if (lane == 0)
+    {
+        part[2 * axis] = hi;
+        part[2 * axis + 1] = lo;
+    }
+}
+
+// The probe's own step from all blocks' sums (SpringNetwork.cpp:156-182), in every block alike, so
+// that no second barrier has to publish it: position and velocity in `prb`, kinetic energy in `ke`.
+__device__ __forceinline__ void probe_step(const Params &p, const float *part, float4 *prb, float *ke)
+{
+    __shared__ float sh_f[3];
+    const int lane = threadIdx.x & 31, axis = threadIdx.x >> 5;
+    if (axis < 3)
+    {
+        float hi = 0.0f, lo = 0.0f;
+        for (unsigned int b = lane; b < gridDim.x; b += 32)
+        {
+            const float2 v = __ldcg(reinterpret_cast<const float2 *>(part + 8 * static_cast<size_t>(b) + 2 * axis));
+            ff_add(hi, lo, v.x, v.y);
+        }
+        warp_ff_sum(hi, lo);
+        if (lane == 0)
+            sh_f[axis] = __fadd_rn(hi, lo);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+        probe_advance(p, sh_f, prb[0], prb[1], *ke);
+    __syncthreads();
+}
+
+template <int SM, int T, bool LEAN>
+__global__ void __launch_bounds__(kStepKernelBlock, kStepMinBlocks) k_run(Params p, int count)
+{
+    Ctl *ctl = p.ctl;
+    if (status_of(ctl) != 0)
+        return; // the same in every block: raised bits reach the status after the last barrier
+    const int sb0 = ctl->sbuf, lb = ctl->lbuf;
+    const bool ext = ctl->ext_pending != 0;
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    constexpr int kPerBlock = kStepKernelBlock / T;
+    __shared__ float4 prb[2]; // the probe's position and velocity
+    __shared__ float probe_ke;
+    const bool probe = !LEAN && p.probe_on;
+    if (probe)
+    {
+        if (threadIdx.x == 0)
+        {
+            prb[0] = ctl->probe_pos;
+            prb[1] = ctl->probe_vel;
+        }
+        __syncthreads();
+    }
+    float e[6];
+    unsigned int gen = 0;
+    int k = 0, go = 1;
+    do
+    {
+#pragma unroll
+        for (int q = 0; q < 6; ++q)
+            e[q] = 0.0f;
+        const int sb = sb0 ^ (k & 1);
+        int pend = particle_step<MODE_STEP, SM, T, true, LEAN, PosShared>(p, g / T, g % T, p.n, sb, lb, ext && k == 0,
+                                                                          prb, e);
+        float *part = p.run_probe + static_cast<size_t>(k & 1) * 8 * gridDim.x; // read until the next step's barrier
+        if (probe)
+        {
+            const int first = blockIdx.x * kPerBlock;
+            probe_block_sum(p, first, min(kPerBlock, p.n - first), part + 8 * static_cast<size_t>(blockIdx.x));
+        }
+        if (!LEAN && p.nbody > 0)
+        {
+            if (!grid_barrier(p.run_arrive, ++gen, 0)) // the bodies read every member's force
+            {
+                go = 0;
+                break;
+            }
+            for (int b = blockIdx.x; b < p.nbody; b += gridDim.x)
+            {
+                pend |= rigid_body_step(p, b, sb);
+                __syncthreads();
+            }
+        }
+        if (pend)
+            atomicOr(&ctl->status_pending, pend);
+        ++k;
+        if (k < count || probe)
+        {
+            go = grid_barrier(p.run_arrive, ++gen, pend);
+            if (probe && go)
+                probe_step(p, part, prb, &probe_ke);
+        }
+    } while (k < count && go == 1);
+    if (go == 0)
+    {
+        if (threadIdx.x == 0)
+            atomicOr(&ctl->status, ST_BARRIER);
+        return;
+    }
+    if (!reduce_energies<6, kStepKernelBlock>(e, p.blk_energy, p.blk_cap, &ctl->done_step, ctl->energies))
+        return;
+    if (threadIdx.x == 0)
+    {
+        publish_energies(ctl);
+        if (probe)
+        {
+            ctl->probe_pos = prb[0];
+            ctl->probe_vel = prb[1];
+            ctl->energies[BS_ENERGY_KINETIC] += static_cast<double>(probe_ke);
+        }
+        ctl->sbuf = sb0 ^ (k & 1);
+        const long long steps = ctl->steps + k;
+        ctl->steps = steps;
+        ctl->rigid_steps = steps;
+        ctl->probe_steps = steps;
+        ctl->ext_pending = 0;
+        *p.run_arrive = 0u; // every block has left its last barrier
+        const int pend = atomicExch(&ctl->status_pending, 0);
+        if (pend)
+            atomicOr(&ctl->status, pend);
+    }
+}
+
+template <int SM> const void *run_fn(int lanes, bool lean)
+{
+    switch (lanes)
+    {
+    case 4:
+        return lean ? reinterpret_cast<const void *>(&k_run<SM, 4, true>) : reinterpret_cast<const void *>(&k_run<SM, 4, false>);
+    case 8:
+        return lean ? reinterpret_cast<const void *>(&k_run<SM, 8, true>) : reinterpret_cast<const void *>(&k_run<SM, 8, false>);
+    case 16:
+        return lean ? reinterpret_cast<const void *>(&k_run<SM, 16, true>)
+                    : reinterpret_cast<const void *>(&k_run<SM, 16, false>);
+    default:
+        return nullptr;
+    }
+}
+
+const void *run_kernel(const Params &p)
+{
+    const bool lean = lean_step(p);
+    switch (p.steric_mode)
+    {
+    case BS_STERIC_LINEAR:
+        return run_fn<BS_STERIC_LINEAR>(p.step_lanes, lean);
+    case BS_STERIC_LJ_12_6_AMBER:
+        return run_fn<BS_STERIC_LJ_12_6_AMBER>(p.step_lanes, lean);
+    case BS_STERIC_LJ_8_6_LEWITT:
+        return run_fn<BS_STERIC_LJ_8_6_LEWITT>(p.step_lanes, lean);
+    case BS_STERIC_LJ_8_6_ZACHARIAS:
+        return run_fn<BS_STERIC_LJ_8_6_ZACHARIAS>(p.step_lanes, lean);
+    default:
+        return nullptr;
+    }
+}
+
+} // namespace
+
+int run_blocks(const Params &p)
+{
+    return static_cast<int>((static_cast<long long>(p.n) * p.step_lanes + kStepKernelBlock - 1) / kStepKernelBlock);
+}
+
+cudaError_t run_fits(const Params &p, bool *fits)
+{
+    *fits = false;
+    const void *fn = run_kernel(p);
+    int dev = 0, sms = 0, coop = 0, per_sm = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess)
+        e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess)
+        e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    if (e != cudaSuccess || !fn || !coop || p.nsys > 0)
+        return e;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kStepKernelBlock, 0);
+    *fits = e == cudaSuccess && run_blocks(p) <= per_sm * sms;
+    return e;
+}
+
+cudaError_t launch_run(const Params &p, int count, cudaStream_t st)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(run_blocks(p)));
+    cfg.blockDim = dim3(kStepKernelBlock);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    void *args[] = {const_cast<Params *>(&p), &count};
+    return cudaLaunchKernelExC(&cfg, run_kernel(p), args);
+}
+
+} // namespace bsg
