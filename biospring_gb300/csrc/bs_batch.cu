@@ -6,10 +6,8 @@
 // search grid (bounding box of its own particles, the single-system formula). Spring partners and
 // pair-list partners are always in the same system.
 //
-// Rebuild: k_batch_bbox (one block per system, then the last block numbers the cells of all
-// systems) -> k_batch_cell_count -> k_batch_cell_scan (one block per system) -> the
-// single-system place / sort / reorder / spring kernels -> k_batch_pairlist (one warp per home
-// particle: systems are sparse, a cell holds a few particles).
+// Rebuild: k_order (bs_order.cu), then k_batch_pairlist (one warp per home particle: systems are
+// sparse, a cell holds a few particles).
 //
 // Step: k_batch_run, a persistent kernel launched with thread-block clusters. A cluster owns a
 // list of whole systems (a host-side longest-processing-time assignment) and runs each of them
@@ -38,168 +36,7 @@ namespace cg = cooperative_groups;
 #ifndef BS_BPL_PREFETCH
 #define BS_BPL_PREFETCH 1
 #endif
-constexpr int kBatchBboxBlock = 256;
 constexpr int kBatchPlWarps = 8;
-constexpr int kMaxSysCells = 1 << 26; // a system spread wider than this falls back to one cell
-
-// One block per system: bounding box of the system's particles and its grid; the last block to
-// finish numbers the cells of all systems and publishes the total as a 1-D grid (gnx = total)
-// for the shared place / sort kernels.
-__global__ void __launch_bounds__(kBatchBboxBlock) k_batch_bbox(Params p)
-{
-    Ctl *ctl = p.ctl;
-    if (status_of(ctl) & kRebuildBlocking)
-        return;
-    const int b = blockIdx.x;
-    const int n0 = p.sys_start[b], n1 = p.sys_start[b + 1];
-    const float4 *pos = p.pos[ctl->sbuf];
-    float v[6] = {FLT_MAX, FLT_MAX, FLT_MAX, FLT_MAX, FLT_MAX, FLT_MAX}; // min x,y,z and -max x,y,z
-    for (int i = n0 + threadIdx.x; i < n1; i += blockDim.x)
-    {
-        const float4 q = pos[i];
-        v[0] = fminf(v[0], q.x);
-        v[1] = fminf(v[1], q.y);
-        v[2] = fminf(v[2], q.z);
-        v[3] = fminf(v[3], -q.x);
-        v[4] = fminf(v[4], -q.y);
-        v[5] = fminf(v[5], -q.z);
-    }
-    __shared__ float sh[6][kBatchBboxBlock / 32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int k = 0; k < 6; ++k)
-    {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            v[k] = fminf(v[k], __shfl_down_sync(0xffffffffu, v[k], o));
-        if (lane == 0)
-            sh[k][warp] = v[k];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-        float mn[3], mx[3];
-        bool ok = n1 > n0;
-        for (int k = 0; k < 3; ++k)
-        {
-            float a = sh[k][0], c = sh[3 + k][0];
-            for (int w = 1; w < kBatchBboxBlock / 32; ++w)
-            {
-                a = fminf(a, sh[k][w]);
-                c = fminf(c, sh[3 + k][w]);
-            }
-            mn[k] = a;
-            mx[k] = -c;
-            ok = ok && isfinite(mn[k]) && isfinite(mx[k]) && mn[k] <= mx[k];
-        }
-        SysGrid g;
-        g.radius = p.list_radius / static_cast<float>(kSparseDiv);
-        int nc[3] = {1, 1, 1};
-        double gmin[3] = {0.0, 0.0, 0.0};
-        double cells = !ok           ? 1.0
-                       : p.lists_off ? free_grid_dims(mn, mx, g.radius, free_cells(n1 - n0), gmin, nc)
-                                     : grid_dims(mn, mx, g.radius, gmin, nc);
-        if (!(cells <= static_cast<double>(kMaxSysCells)))
-        {
-            // one cell holds the whole system: the neighbour walk sees every particle, which
-            // gives the same pairs (every candidate is tested against the list radius)
-            nc[0] = nc[1] = nc[2] = 1;
-            cells = 1.0;
-        }
-        for (int k = 0; k < 3; ++k)
-            g.gmin[k] = gmin[k];
-        g.nx = nc[0];
-        g.ny = nc[1];
-        g.nz = nc[2];
-        g.cells = static_cast<int>(cells);
-        p.sys_grid[b] = g;
-        p.stale_at[b] = LLONG_MAX; // a fresh list
-        p.sys_status[b] &= ~ST_STALE;
-    }
-    __threadfence();
-    __syncthreads();
-    __shared__ bool last;
-    if (threadIdx.x == 0)
-        last = atomicAdd(&ctl->done_bbox, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (!last || threadIdx.x != 0)
-        return;
-    __threadfence();
-    long long total = 0;
-    for (int s = 0; s < p.nsys; ++s)
-    {
-        p.sys_cells[s] = static_cast<int>(total < INT_MAX ? total : INT_MAX);
-        total += __ldcg(&p.sys_grid[s].cells);
-    }
-    p.sys_cells[p.nsys] = static_cast<int>(total < INT_MAX ? total : INT_MAX);
-    if (total > static_cast<long long>(p.cell_cap))
-    {
-        ctl->ncells_needed = static_cast<int>(total < INT_MAX ? total : INT_MAX);
-        atomicOr(&ctl->status, ST_CELL_CAPACITY);
-    }
-    ctl->gnx = static_cast<int>(total < p.cell_cap ? total : p.cell_cap);
-    ctl->gny = 1;
-    ctl->gnz = 1;
-    atomicAnd(&ctl->status, ~ST_STALE);
-    ctl->done_bbox = 0u;
-}
-
-__global__ void __launch_bounds__(kBuildBlock) k_batch_cell_count(Params p)
-{
-    Ctl *ctl = p.ctl;
-    if (status_of(ctl) & kRebuildBlocking)
-        return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.n)
-        return;
-    const int b = p.sys_of[i];
-    const SysGrid &g = p.sys_grid[b];
-    const float4 q = p.pos[ctl->sbuf][i];
-    const int cx = ref_cell_coord(q.x, g.gmin[0], g.radius, g.nx);
-    const int cy = ref_cell_coord(q.y, g.gmin[1], g.radius, g.ny);
-    const int cz = ref_cell_coord(q.z, g.gmin[2], g.radius, g.nz);
-    const int c = p.sys_cells[b] + cx + cy * g.nx + cz * g.nx * g.ny;
-    p.cell_of[i] = c;
-    atomicAdd(&p.cell_cnt[c], 1);
-}
-
-// One block per system: exclusive scan of the system's cell counts, offset by the system's first
-// slot; primes the fill cursors and clears the counts for the next rebuild.
-__global__ void __launch_bounds__(1024) k_batch_cell_scan(Params p)
-{
-    Ctl *ctl = p.ctl;
-    if (status_of(ctl) & kRebuildBlocking)
-        return;
-    const int b = blockIdx.x;
-    const int c0 = p.sys_cells[b], c1 = p.sys_cells[b + 1];
-    const int nc = c1 - c0;
-    const int per = (nc + blockDim.x - 1) / blockDim.x;
-    const int b0 = c0 + threadIdx.x * per, b1 = min(c1, b0 + per);
-    int sum = 0;
-    for (int c = b0; c < b1; ++c)
-        sum += p.cell_cnt[c];
-    __shared__ int sh[1024];
-    sh[threadIdx.x] = sum;
-    __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1)
-    {
-        const int v = threadIdx.x >= o ? sh[threadIdx.x - o] : 0;
-        __syncthreads();
-        sh[threadIdx.x] += v;
-        __syncthreads();
-    }
-    int run = p.sys_start[b] + sh[threadIdx.x] - sum;
-    for (int c = b0; c < b1; ++c)
-    {
-        const int k = p.cell_cnt[c];
-        p.cell_start[c] = run;
-        p.cell_fill[c] = run;
-        p.cell_cnt[c] = 0;
-        run += k;
-    }
-    if (threadIdx.x == 0)
-        p.cell_start[c1] = p.sys_start[b + 1];
-}
 
 // Typed pair lists, one warp per home particle: the rules of the cell-block build (every pair
 // within the list radius of its term, the slot itself and spring partners excluded, static
@@ -631,14 +468,6 @@ __global__ void __launch_bounds__(256) k_batch_finish(Params p, int chunk)
 }
 
 } // namespace
-
-int launch_batch_grid(const Params &p, cudaStream_t st)
-{
-    k_batch_bbox<<<p.nsys, kBatchBboxBlock, 0, st>>>(p);
-    k_batch_cell_count<<<(p.n + kBuildBlock - 1) / kBuildBlock, kBuildBlock, 0, st>>>(p);
-    k_batch_cell_scan<<<p.nsys, 1024, 0, st>>>(p);
-    return 3;
-}
 
 int launch_batch_pairlist(const Params &p, cudaStream_t st)
 {

@@ -95,7 +95,7 @@ struct bs_sim
     long long launches = 0;
     // growable buffers (pair lists, grid arrays), freed on regrowth
     unsigned int *pl_idx[kLists] = {nullptr, nullptr, nullptr, nullptr};
-    int *cell_buf[4] = {nullptr, nullptr, nullptr, nullptr};
+    int *cell_buf[2] = {nullptr, nullptr};
     // batched ensembles: caller's partition into systems (empty: one system)
     std::vector<int64_t> sys_off;
     BatchShape shape{256, 4, 1};
@@ -249,7 +249,7 @@ void free_growable(bs_sim *s)
             cudaFree(s->pl_idx[t]);
         s->pl_idx[t] = nullptr;
     }
-    for (int k = 0; k < 4; ++k)
+    for (int k = 0; k < 2; ++k)
     {
         if (s->cell_buf[k])
             cudaFree(s->cell_buf[k]);
@@ -274,15 +274,11 @@ int alloc_lists(bs_sim *s, const int caps[kLists], int cell_cap)
         p.pl[t].idx = s->pl_idx[t];
         p.pl[t].cap = cap;
     }
-    for (int k = 0; k < 3; ++k)
+    for (int k = 0; k < 2; ++k)
         BS_CUDA(cudaMalloc(reinterpret_cast<void **>(&s->cell_buf[k]), (static_cast<size_t>(cell_cap) + 1) * sizeof(int)));
     BS_CUDA(cudaMemsetAsync(s->cell_buf[0], 0, (static_cast<size_t>(cell_cap) + 1) * sizeof(int), s->stream));
-    BS_CUDA(cudaMalloc(reinterpret_cast<void **>(&s->cell_buf[3]),
-                       (static_cast<size_t>(cell_cap) / kScanTile + 2) * sizeof(int)));
     p.cell_cnt = s->cell_buf[0];
     p.cell_start = s->cell_buf[1];
-    p.cell_fill = s->cell_buf[2];
-    p.tile_sum = s->cell_buf[3];
     p.cell_cap = cell_cap;
     destroy_graph(s);
     return BS_OK;
@@ -1132,6 +1128,10 @@ int bs_setup(bs_sim *s, const bs_config *cfg)
         BS_CUDA(s->dev.alloc(&p.pl[t].cnt, npad));
     BS_CUDA(s->dev.alloc(&p.cell_of, npad));
     BS_CUDA(s->dev.alloc(&p.tmp_key, npad));
+    BS_CUDA(s->dev.alloc(&p.cell_at, npad));
+    BS_CUDA(s->dev.alloc(&p.tile_sum, kOrderMaxBlocks));
+    BS_CUDA(s->dev.alloc(&p.order_sync, 2));
+    BS_CUDA(cudaMemsetAsync(p.order_sync, 0, 2 * sizeof(unsigned int), s->stream));
     s->step_blocks = static_cast<int>((static_cast<long long>(p.n) * 16 + kStepBlock - 1) / kStepBlock);
     p.blk_cap = s->step_blocks;
     BS_CUDA(s->dev.alloc(&p.blk_energy, energy_scratch_doubles(s->step_blocks)));
@@ -1231,6 +1231,11 @@ int bs_setup(bs_sim *s, const bs_config *cfg)
         p.sys_of = d_of;
         BS_CUDA(s->dev.alloc(&p.sys_grid, nsys));
         BS_CUDA(s->dev.alloc(&p.sys_cells, nsys + 1));
+        std::vector<unsigned int> box(6 * static_cast<size_t>(nsys)); // empty boxes
+        for (size_t k = 0; k < box.size(); ++k)
+            box[k] = k % 6 < 3 ? 0xffffffffu : 0u;
+        BS_CUDA(s->dev.alloc(&p.sys_box, box.size()));
+        BS_CUDA(cudaMemcpy(p.sys_box, box.data(), sizeof(unsigned int) * box.size(), cudaMemcpyHostToDevice));
         BS_CUDA(s->dev.alloc(&p.sys_status, nsys));
         BS_CUDA(s->dev.alloc(&p.sys_steps, nsys));
         BS_CUDA(s->dev.alloc(&p.stale_at, nsys));
@@ -1477,6 +1482,7 @@ int bs_setup(bs_sim *s, const bs_config *cfg)
     p.k_imp_f = static_cast<float>(kImpForceConvert);
     p.k_hydro_e = static_cast<float>(kAvogadro * 1.0E-3);
 
+    BS_CUDA(order_blocks(p, &p.order_blocks));
     bool fits = false;
     BS_CUDA(run_fits(p, &fits));
     if (fits)

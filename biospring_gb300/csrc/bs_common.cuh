@@ -78,9 +78,7 @@ struct Ctl
     int status;
     int sbuf;                 // index of the buffer holding the current positions/velocities
     int lbuf;                 // index of the buffer holding the current particle layout
-    unsigned int done_step;   // last-block counters
-    unsigned int done_bbox;
-    unsigned int done_reorder;
+    unsigned int done_step;   // last-block counter of the step kernel
     long long steps;          // completed steps since setup
     int max_row[kLists];      // largest row of each pair list seen at the last build
     int ncells_needed;
@@ -192,10 +190,12 @@ struct Params
     int *cell_of;             // [npad] cell of each sorted slot (new layout)
     int *cell_cnt;            // [cell_cap + 1]
     int *cell_start;          // [cell_cap + 1]
-    int *cell_fill;           // [cell_cap]
-    unsigned long long *tmp_key; // [npad] cell-sort key of each placed particle (x bits, caller id)
+    unsigned long long *tmp_key; // [npad] order key of each placed particle (x bits, caller id)
     int cell_cap;
-    int *tile_sum;            // [cell_cap / kScanTile + 2] per-tile totals of the cell scan
+    int2 *cell_at;            // [npad] cell of each particle in the old order, its place of arrival there
+    int *tile_sum;            // [kOrderMaxBlocks] cell totals of each block's share in the cell scan
+    unsigned int *order_sync; // [2] k_order's grid-barrier word and count of finished blocks, 0 between launches
+    int order_blocks;         // its grid, resident at once
     int pl_sparse;            // build the pair lists one warp per particle (few particles per cell)
     int lists_off;            // no nonbonded term is on: no pair lists, the grid only orders the particles
     int coul_all;             // list Coulomb partners of every dynamic particle, charged or not (charge gradients)
@@ -235,6 +235,7 @@ struct Params
     const int *sys_start;     // [nsys + 1] slot ranges
     const int *sys_of;        // [npad] system of each slot (0 for padding)
     SysGrid *sys_grid;        // [nsys]
+    unsigned int *sys_box;    // [nsys * 6] order-preserving codes of each system's box (reset after use)
     int *sys_cells;           // [nsys + 1] first global cell of each system
     int *sys_status;          // [nsys] ST_NONFINITE / ST_STALE raised by the system
     long long *sys_steps;     // [nsys] steps completed by each system
@@ -278,9 +279,9 @@ struct Params
 constexpr int kMaxCluster = 16;
 
 // Systems without nonbonded terms: particles per cell the host aims at, and the cells a system of
-// n particles may have. A cell is ranked by one warp (k_cell_sort) in time quadratic in its
-// particles: with the whole system in one cell a rebuild of 20,000 particles took 117 ms, with 8 a
-// cell the sort takes a few microseconds.
+// n particles may have. A particle is ranked within its cell by counting (k_order), so the sort's time goes
+// with the particles a cell holds: the whole system in one cell is quadratic (117 ms a rebuild at 20,000
+// particles with one warp a cell).
 constexpr double kFreeCell = 8.0;
 __host__ __device__ constexpr double free_cells(double n) { return 4.0 * n + 64.0; }
 

@@ -18,8 +18,7 @@
 // then needs only 1/r^2 (no square root, no division).
 //
 // Rebuild (every K steps, or when a particle drifted more than skin/2):
-//   k_bbox -> k_cell_count -> k_cell_scan -> k_cell_place -> k_cell_sort -> k_reorder
-//   -> k_spring_ell -> k_pairlist
+//   k_order (bs_order.cu) -> k_pairlist, or k_batch_pairlist (bs_batch.cu) for sparse systems
 // Step: k_step, T consecutive lanes per particle, gathers its springs and nonbonded pairs (no
 // atomics on forces, so results are deterministic) and integrates in the same pass.
 //
@@ -41,390 +40,6 @@ namespace bsg
 
 namespace
 {
-
-// ------------------------------------------------------------------------------------------
-// Rebuild kernels
-// ------------------------------------------------------------------------------------------
-
-__global__ void __launch_bounds__(kBboxBlock) k_bbox(Params p)
-{
-    pdl_enter();
-    Ctl *ctl = p.ctl;
-    if (status_of(ctl) & kRebuildBlocking)
-        return;
-    const float4 *pos = p.pos[ctl->sbuf];
-    float v[6] = {FLT_MAX, FLT_MAX, FLT_MAX, FLT_MAX, FLT_MAX, FLT_MAX}; // min x,y,z and -max x,y,z
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < p.n; i += gridDim.x * blockDim.x)
-    {
-        const float4 q = pos[i];
-        v[0] = fminf(v[0], q.x);
-        v[1] = fminf(v[1], q.y);
-        v[2] = fminf(v[2], q.z);
-        v[3] = fminf(v[3], -q.x);
-        v[4] = fminf(v[4], -q.y);
-        v[5] = fminf(v[5], -q.z);
-    }
-    __shared__ float sh[6][kBboxBlock / 32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int k = 0; k < 6; ++k)
-    {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            v[k] = fminf(v[k], __shfl_down_sync(0xffffffffu, v[k], o));
-        if (lane == 0)
-            sh[k][warp] = v[k];
-    }
-    __syncthreads();
-    unsigned int *enc = ctl->bbox_enc;
-    if (threadIdx.x < 6)
-    {
-        float m = sh[threadIdx.x][0];
-        for (int w = 1; w < kBboxBlock / 32; ++w)
-            m = fminf(m, sh[threadIdx.x][w]);
-        if (threadIdx.x < 3)
-            atomicMin(&enc[threadIdx.x], f2ord(m));
-        else
-            atomicMax(&enc[threadIdx.x], f2ord(-m));
-    }
-    __threadfence();
-    __syncthreads();
-    __shared__ bool last;
-    if (threadIdx.x == 0)
-        last = atomicAdd(&ctl->done_bbox, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (!last || threadIdx.x != 0)
-        return;
-    __threadfence();
-    float mn[3], mx[3];
-    for (int k = 0; k < 3; ++k)
-    {
-        mn[k] = ord2f(atomicAdd(&enc[k], 0u));
-        mx[k] = ord2f(atomicAdd(&enc[3 + k], 0u));
-        enc[k] = 0xffffffffu; // reset for the next rebuild
-        enc[3 + k] = 0u;
-    }
-    // the cell-block list build uses cells of a kGridDiv-th of the list radius, the warp-per-particle
-    // build (sparse systems) cells of the list radius
-    float edge = p.list_radius / static_cast<float>(p.pl_sparse ? kSparseDiv : kGridDiv);
-    int nc[3];
-    double gmin[3];
-    const double cells = p.lists_off ? free_grid_dims(mn, mx, edge, free_cells(p.n), gmin, nc)
-                                     : grid_dims(mn, mx, edge, gmin, nc);
-    for (int k = 0; k < 3; ++k)
-        ctl->gmin[k] = gmin[k];
-    ctl->gradius = edge;
-    ctl->gnx = nc[0];
-    ctl->gny = nc[1];
-    ctl->gnz = nc[2];
-    if (!(cells <= static_cast<double>(p.cell_cap)))
-    {
-        ctl->ncells_needed = cells < 2.0e9 ? static_cast<int>(cells) : INT_MAX;
-        atomicOr(&ctl->status, ST_CELL_CAPACITY);
-    }
-    if (status_of(ctl) & ST_STALE)
-        ctl->stale_events += 1;
-    atomicAnd(&ctl->status, ~ST_STALE);
-    ctl->done_bbox = 0u;
-}
-
-__global__ void __launch_bounds__(kBuildBlock) k_cell_count(Params p)
-{
-    pdl_enter();
-    Ctl *ctl = p.ctl;
-    if (status_of(ctl) & kRebuildBlocking)
-        return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.n)
-        return;
-    const float4 q = p.pos[ctl->sbuf][i];
-    const float r = ctl->gradius;
-    const int nx = ctl->gnx, ny = ctl->gny, nz = ctl->gnz;
-    const int cx = ref_cell_coord(q.x, ctl->gmin[0], r, nx);
-    const int cy = ref_cell_coord(q.y, ctl->gmin[1], r, ny);
-    const int cz = ref_cell_coord(q.z, ctl->gmin[2], r, nz);
-    const int c = cx + cy * nx + cz * nx * ny;
-    p.cell_of[i] = c;
-    atomicAdd(&p.cell_cnt[c], 1);
-}
-
-// Exclusive scan of the cell counts in three passes over tiles of kScanTile cells, so that grids
-// of millions of (mostly empty) cells cost a few microseconds. Pass 1: each block scans one tile
-// (4 consecutive cells per thread) and writes the in-tile prefixes and the tile's total.
-__global__ void __launch_bounds__(1024) k_scan_tiles(Params p)
-{
-    pdl_enter();
-    Ctl *ctl = p.ctl;
-    if (status_of(ctl) & kRebuildBlocking)
-        return;
-    const int nc = ctl->gnx * ctl->gny * ctl->gnz;
-    const int base = blockIdx.x * kScanTile;
-    if (base >= nc)
-        return;
-    const int c0 = base + 4 * threadIdx.x;
-    int v[4], sum = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-    {
-        v[k] = c0 + k < nc ? p.cell_cnt[c0 + k] : 0;
-        sum += v[k];
-    }
-    __shared__ int sh_warp[32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int inc = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1)
-    {
-        const int t = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o)
-            inc += t;
-    }
-    if (lane == 31)
-        sh_warp[warp] = inc;
-    __syncthreads();
-    if (warp == 0)
-    {
-        int w = sh_warp[lane];
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1)
-        {
-            const int t = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o)
-                w += t;
-        }
-        sh_warp[lane] = w; // inclusive over warps
-    }
-    __syncthreads();
-    int run = inc - sum + (warp > 0 ? sh_warp[warp - 1] : 0);
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-    {
-        if (c0 + k < nc)
-            p.cell_start[c0 + k] = run;
-        run += v[k];
-    }
-    if (threadIdx.x == blockDim.x - 1)
-        p.tile_sum[blockIdx.x] = sh_warp[31];
-}
-
-// Pass 2 (one block): exclusive scan of the tile totals, in place; writes the grand total after
-// the last cell.
-__global__ void __launch_bounds__(1024) k_scan_top(Params p)
-{
-    pdl_enter();
-    Ctl *ctl = p.ctl;
-    if (status_of(ctl) & kRebuildBlocking)
-        return;
-    const int nc = ctl->gnx * ctl->gny * ctl->gnz;
-    const int nt = (nc + kScanTile - 1) / kScanTile;
-    const int per = (nt + blockDim.x - 1) / blockDim.x;
-    const int b0 = threadIdx.x * per, b1 = min(nt, b0 + per);
-    int sum = 0;
-    for (int t = b0; t < b1; ++t)
-        sum += p.tile_sum[t];
-    __shared__ int sh[1024];
-    sh[threadIdx.x] = sum;
-    __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1)
-    {
-        const int v = threadIdx.x >= o ? sh[threadIdx.x - o] : 0;
-        __syncthreads();
-        sh[threadIdx.x] += v;
-        __syncthreads();
-    }
-    int run = sh[threadIdx.x] - sum;
-    for (int t = b0; t < b1; ++t)
-    {
-        const int k = p.tile_sum[t];
-        p.tile_sum[t] = run;
-        run += k;
-    }
-    if (threadIdx.x == blockDim.x - 1)
-        p.cell_start[nc] = run;
-}
-
-// Pass 3: adds each tile's offset, primes the fill cursors and clears the counts for the next
-// rebuild.
-__global__ void __launch_bounds__(1024) k_scan_add(Params p)
-{
-    pdl_enter();
-    Ctl *ctl = p.ctl;
-    if (status_of(ctl) & kRebuildBlocking)
-        return;
-    const int nc = ctl->gnx * ctl->gny * ctl->gnz;
-    const int base = blockIdx.x * kScanTile;
-    if (base >= nc)
-        return;
-    const int off = p.tile_sum[blockIdx.x];
-    const int c0 = base + 4 * threadIdx.x;
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-    {
-        const int c = c0 + k;
-        if (c < nc)
-        {
-            const int st = p.cell_start[c] + off;
-            p.cell_start[c] = st;
-            p.cell_fill[c] = st;
-            p.cell_cnt[c] = 0;
-        }
-    }
-}
-
-__global__ void __launch_bounds__(kBuildBlock) k_cell_place(Params p)
-{
-    pdl_enter();
-    Ctl *ctl = p.ctl;
-    if (status_of(ctl) & kRebuildBlocking)
-        return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.n)
-        return;
-    const int slot = atomicAdd(&p.cell_fill[p.cell_of[i]], 1);
-    const int id = p.perm[ctl->lbuf][i];
-    // the order key of k_cell_sort: x coordinate, then caller id
-    p.tmp_key[slot] = (static_cast<unsigned long long>(f2ord(p.pos[ctl->sbuf][i].x)) << 32) |
-                      static_cast<unsigned int>(id);
-}
-
-// One warp per cell: orders the cell's particles by x coordinate, ties by caller id, which makes
-// the layout deterministic and every x-run of cells one x-sorted sequence (the pair-list build
-// bounds its candidates in a run by binary search). Cells are filled in any order by
-// k_cell_place; the reference appends to a cell in index order (nsearch.hpp:376-389), an order
-// no result here depends on.
-__global__ void __launch_bounds__(kBuildBlock) k_cell_sort(Params p)
-{
-    pdl_enter();
-    Ctl *ctl = p.ctl;
-    if (status_of(ctl) & kRebuildBlocking)
-        return;
-    const int nc = ctl->gnx * ctl->gny * ctl->gnz;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    int *out = p.perm[ctl->lbuf ^ 1];
-    const unsigned long long *__restrict__ key = p.tmp_key;
-    for (int c = warp; c < nc; c += nwarps)
-    {
-        const int s0 = p.cell_start[c], s1 = p.cell_start[c + 1];
-        const int len = s1 - s0;
-        if (len <= 64)
-        {
-            // up to two keys per lane, ranked against every key of the cell by shuffles
-            const unsigned long long k0 = lane < len ? key[s0 + lane] : ~0ull;
-            const unsigned long long k1 = lane + 32 < len ? key[s0 + 32 + lane] : ~0ull;
-            int r0 = 0, r1 = 0;
-            for (int f = 0; f < len; ++f)
-            {
-                const unsigned long long kf = __shfl_sync(0xffffffffu, f < 32 ? k0 : k1, f & 31);
-                r0 += kf < k0;
-                r1 += kf < k1;
-            }
-            if (lane < len)
-            {
-                out[s0 + r0] = static_cast<int>(k0 & 0xffffffffu);
-                p.cell_of[s0 + r0] = c;
-            }
-            if (lane + 32 < len)
-            {
-                out[s0 + r1] = static_cast<int>(k1 & 0xffffffffu);
-                p.cell_of[s0 + r1] = c;
-            }
-            continue;
-        }
-        for (int e = lane; e < len; e += 32)
-        {
-            const unsigned long long ke = key[s0 + e];
-            int rank = 0;
-            for (int f = 0; f < len; ++f)
-                rank += key[s0 + f] < ke;
-            out[s0 + rank] = static_cast<int>(ke & 0xffffffffu);
-            p.cell_of[s0 + rank] = c;
-        }
-    }
-}
-
-// Moves the state into the new layout, records build positions and the new inverse permutation,
-// then (last block) makes the new layout current.
-__global__ void __launch_bounds__(kBuildBlock) k_reorder(Params p)
-{
-    pdl_enter();
-    Ctl *ctl = p.ctl;
-    if (status_of(ctl) & kRebuildBlocking)
-        return;
-    const int sb = ctl->sbuf, lb = ctl->lbuf;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < p.n)
-    {
-        const int id = p.perm[lb ^ 1][i];
-        const int old = p.inv[id];
-        const float4 q = p.pos[sb][old];
-        p.pos[sb ^ 1][i] = q;
-        p.vel[sb ^ 1][i] = p.vel[sb][old];
-        if (p.pos_lo[0])
-            p.pos_lo[sb ^ 1][i] = p.pos_lo[sb][old];
-        p.fhi[lb ^ 1][i] = p.fhi[lb][old];
-        p.chg[lb ^ 1][i] = p.chg[lb][old];
-        p.hyd[lb ^ 1][i] = p.hyd[lb][old];
-        if (p.bur[0])
-            p.bur[lb ^ 1][i] = p.bur[lb][old];
-        p.flags[lb ^ 1][i] = p.flags[lb][old];
-        p.iprm[lb ^ 1][i] = p.iprm[lb][old];
-        p.pos_build[i] = q;
-        p.inv[id] = i;
-    }
-    __threadfence();
-    __syncthreads();
-    __shared__ bool last;
-    if (threadIdx.x == 0)
-        last = atomicAdd(&ctl->done_reorder, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (last && threadIdx.x == 0)
-    {
-        ctl->sbuf = sb ^ 1;
-        ctl->lbuf = lb ^ 1;
-        ctl->done_reorder = 0u;
-    }
-}
-
-// Springs of every slot in the new layout, partners as slots (ELL, column-major). ell_lanes
-// consecutive threads share a slot and take every ell_lanes-th spring of its caller-order row,
-// so the row is read with contiguous loads and the partner lookups of a slot overlap; with one
-// lane per slot, the threads of a warp store each column contiguously.
-__global__ void __launch_bounds__(kBuildBlock) k_spring_ell(Params p)
-{
-    pdl_enter();
-    Ctl *ctl = p.ctl;
-    if (status_of(ctl) & kRebuildBlocking)
-        return;
-    const long long g = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const int L = p.ell_lanes;
-    const int s = static_cast<int>(g / L), t = static_cast<int>(g % L);
-    if (s >= p.npad)
-        return;
-    if (s >= p.n)
-    {
-        if (t == 0)
-            p.se_deg[s] = 0;
-        return;
-    }
-    const int id = p.perm[ctl->lbuf][s];
-    const int r0 = p.sp_row[id], r1 = p.sp_row[id + 1];
-    const size_t stride = static_cast<size_t>(p.npad);
-    for (int e = r0 + t; e < r1; e += L)
-    {
-        const unsigned int c = p.sp_col[e];
-        const unsigned int slot = static_cast<unsigned int>(p.inv[c & kSlotMask]);
-        const size_t dst = static_cast<size_t>(e - r0) * stride + s;
-        p.se_col[dst] = slot | (c & ~kSlotMask);
-        p.se_k[dst] = p.sp_k[e];
-        p.se_r0[dst] = p.sp_r0[e];
-        if (p.se_sid)
-            p.se_sid[dst] = p.sp_sid[e];
-    }
-    if (t == 0)
-        p.se_deg[s] = r1 - r0;
-}
 
 // Typed pair lists from the cell grid: steric (every pair within its cutoff + skin, dynamic and
 // static partners apart), Coulomb (both charged) and hydrophobic (both hydrophobic), minus the
@@ -1196,29 +811,8 @@ static void launch_chain(void (*kern)(KArgs...), unsigned grid, unsigned block, 
 
 int launch_rebuild(const Params &p, cudaStream_t st)
 {
-    const int nb = (p.n + kBuildBlock - 1) / kBuildBlock;
-    int bb = (p.n + kBboxBlock - 1) / kBboxBlock;
-    bb = bb > 304 ? 304 : (bb < 1 ? 1 : bb);
-    int launched = 0;
-    if (p.nsys > 0)
-        launched += launch_batch_grid(p, st);
-    else
-    {
-        const int tiles = p.cell_cap / kScanTile + 1;
-        launch_chain(k_bbox, bb, kBboxBlock, 0, st, p);
-        launch_chain(k_cell_count, nb, kBuildBlock, 0, st, p);
-        launch_chain(k_scan_tiles, tiles, 1024, 0, st, p);
-        launch_chain(k_scan_top, 1, 1024, 0, st, p);
-        launch_chain(k_scan_add, tiles, 1024, 0, st, p);
-        launched += 5;
-    }
-    launch_chain(k_cell_place, nb, kBuildBlock, 0, st, p);
-    launch_chain(k_cell_sort, 1216, kBuildBlock, 0, st, p);
-    launch_chain(k_reorder, nb, kBuildBlock, 0, st, p);
-    launch_chain(k_spring_ell,
-                 static_cast<unsigned>((static_cast<long long>(p.npad) * p.ell_lanes + kBuildBlock - 1) / kBuildBlock),
-                 kBuildBlock, 0, st, p);
-    launched += 4;
+    launch_order(p, st);
+    int launched = 1;
     if (p.lists_off)
         return launched;
     if (p.nsys > 0 || p.pl_sparse)

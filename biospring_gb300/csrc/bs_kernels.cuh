@@ -19,7 +19,10 @@ constexpr int kStepKernelBlock = BS_STEP_BLOCK;
 constexpr int kStepMinBlocks = BS_STEP_MIN_BLOCKS;
 constexpr int kBuildBlock = 128;
 constexpr int kBuildLanes = 8;    // threads per slot of the spring-table rebuild when the table fits L2
-constexpr int kBboxBlock = 256;
+// k_order: most blocks of its grid, and the threads a particle it is sized for (small systems use as few
+// blocks as their spring table needs, for cheaper barriers)
+constexpr int kOrderMaxBlocks = 1024;
+constexpr int kOrderLanes = 8;
 constexpr int kMaxEnergyBlocks = 1 << 16;
 
 // status bits that stop a rebuild; a stale list is what a rebuild repairs
@@ -86,7 +89,6 @@ constexpr int kPlStage = BS_PL_STAGE; // candidate positions staged in shared me
 constexpr int kPlMinBlocks = 4;       // resident list-build blocks per SM (the stage allows 4)
 constexpr int kPlBatch = 16;         // home particles per warp
 constexpr int kPlBatchesPerCell = 4; // warps per cell (a cell with more than 64 particles loops)
-constexpr int kScanTile = 4096;      // cells per block of the cell-count scan (4 per thread)
 
 enum StepMode
 {
@@ -96,6 +98,8 @@ enum StepMode
 
 // Launchers (all asynchronous on `stream`); each returns the number of kernels launched.
 int launch_rebuild(const Params &p, cudaStream_t stream);
+cudaError_t launch_order(const Params &p, cudaStream_t stream); // bs_order.cu
+cudaError_t order_blocks(const Params &p, int *blocks);
 int launch_step(const Params &p, int mode, cudaStream_t stream);      // step kernel, then the bodies
 int launch_step_only(const Params &p, int mode, cudaStream_t stream); // the step kernel alone
 int launch_rigid(const Params &p, cudaStream_t stream);               // bs_rigid.cu
@@ -155,7 +159,6 @@ struct BatchShape
     int lanes;   // threads per particle (1, 2, 4, 8)
     int cluster; // blocks per cluster (1, 2, 4, 8)
 };
-int launch_batch_grid(const Params &p, cudaStream_t stream);
 int launch_batch_pairlist(const Params &p, cudaStream_t stream);
 cudaError_t launch_batch_run(const Params &p, const BatchShape &shape, int chunk, cudaStream_t stream);
 int launch_batch_finish(const Params &p, int chunk, cudaStream_t stream);

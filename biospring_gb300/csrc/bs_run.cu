@@ -24,33 +24,6 @@ namespace
 
 static_assert(kRigidBlock == kStepKernelBlock, "k_run's blocks serve the bodies");
 
-// All blocks of the (cooperative) grid meet; gen counts the meetings of this launch from 1. Returns 1,
-// or 2 in every block alike if a thread of any block came with `pend` set, or 0 if this block gave the
-// (bounded) wait up: the others then do so too, and the launch ends without advancing the state.
-// Two flag bits, by the parity of gen: a block may already be at the next meeting when another reads
-// the word, but never two ahead.
-constexpr unsigned int kRunCount = (1u << 30) - 1u;
-__device__ __forceinline__ int grid_barrier(unsigned int *arrive, unsigned int gen, int pend)
-{
-    __shared__ int met;
-    const int any = __syncthreads_or(pend);
-    if (threadIdx.x == 0)
-    {
-        const unsigned int want = gen * gridDim.x, flag = 1u << (30 + (gen & 1u));
-        if (any)
-            atomicOr(arrive, flag);
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrive) : "memory");
-        unsigned int seen = 0;
-        int tries = 0;
-        do
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(arrive) : "memory");
-        while ((seen & kRunCount) < want && ++tries < kRunSpinLimit);
-        met = (seen & kRunCount) < want ? 0 : ((seen & flag) ? 2 : 1);
-    }
-    __syncthreads();
-    return met;
-}
-
 // The probe's sum over this block's particles, (hi, lo) per axis, into the block's row of `part`.
 __device__ __forceinline__ void probe_block_sum(const Params &p, const int first, const int count, float *part)
 {
