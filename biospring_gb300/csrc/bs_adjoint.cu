@@ -52,9 +52,9 @@ __device__ __forceinline__ void hvp(float phi, float dphi, float inv, float ux, 
 // device's Coulomb constant: dL/dq_s += (phi / q_s) u.(nu_s - nu_j), and the same with phi / q_j for
 // a static partner, which has no row of its own (added atomically). The rows list every partner
 // of the slot when charge gradients are asked for, so uncharged particles get theirs too.
-template <int T>
-__device__ __forceinline__ void adj_coulomb(const Params &p, const AdjState &a, int s, int t, int lb, float4 xi,
-                                            float4 ni, float qs, float &hx, float &hy, float &hz, float &gqs)
+template <int T, class NU>
+__device__ __forceinline__ void adj_coulomb(const Params &p, const AdjState &a, const NU nu, int s, int t, int lb,
+                                            float4 xi, float4 ni, float qs, float &hx, float &hy, float &hz, float &gqs)
 {
     const PairList &L = p.pl[1];
     const int cnt = L.cnt[s];
@@ -81,7 +81,7 @@ __device__ __forceinline__ void adj_coulomb(const Params &p, const AdjState &a, 
         const float phi = per_s * qs;
         const float dphi = (dist ? -3.0f : -2.0f) * phi * inv;
         const float ux = dx * inv, uy = dy * inv, uz = dz * inv;
-        const float4 nj = st ? make_float4(0.f, 0.f, 0.f, 0.f) : a.nu_in[j];
+        const float4 nj = st ? make_float4(0.f, 0.f, 0.f, 0.f) : nu[j];
         if (phi != 0.0f)
             hvp(phi, dphi, inv, ux, uy, uz, nj.x - ni.x, nj.y - ni.y, nj.z - ni.z, hx, hy, hz);
         if (a.gq)
@@ -131,9 +131,9 @@ __device__ __forceinline__ bool spring_geometry(float4 xi, float4 xj, float4 li,
 }
 
 // Linear steric overlaps of slot s from one pair list, lane t of T.
-template <int T, int KIND>
-__device__ __forceinline__ void adj_steric(const Params &p, const AdjState &a, int s, int t, float4 xi, float4 ni,
-                                           float &hx, float &hy, float &hz)
+template <int T, int KIND, class NU>
+__device__ __forceinline__ void adj_steric(const Params &p, const AdjState &a, const NU nu, int s, int t, float4 xi,
+                                           float4 ni, float &hx, float &hy, float &hz)
 {
     const PairList &L = p.pl[KIND == 2 ? kListStericStatic : 0];
     const int cnt = L.cnt[s];
@@ -156,9 +156,60 @@ __device__ __forceinline__ void adj_steric(const Params &p, const AdjState &a, i
         if (dv > 0.0f)
             continue;
         const float inv = 1.0f / d;
-        const float4 nj = KIND == 2 ? make_float4(0.f, 0.f, 0.f, 0.f) : a.nu_in[j];
+        const float4 nj = KIND == 2 ? make_float4(0.f, 0.f, 0.f, 0.f) : nu[j];
         hvp(cs * dv, cs, inv, dx * inv, dy * inv, dz * inv, nj.x - ni.x, nj.y - ni.y, nj.z - ni.z, hx, hy, hz);
     }
+}
+
+// Nonbonded terms of one backward step for slot s, lane t of T.
+template <int T, class NU>
+__device__ __forceinline__ void adj_nonbonded(const Params &p, const AdjState &a, const NU nu, int s, int t, int lb,
+                                              float4 xi, float4 ni, float &hx, float &hy, float &hz, float &gqs)
+{
+    if (p.steric_on)
+    {
+        if (p.pl16)
+            adj_steric<T, 0>(p, a, nu, s, t, xi, ni, hx, hy, hz);
+        else
+            adj_steric<T, 1>(p, a, nu, s, t, xi, ni, hx, hy, hz);
+        if (p.pl[kListStericStatic].on && p.pl[kListStericStatic].cnt[s] > 0)
+            adj_steric<T, 2>(p, a, nu, s, t, xi, ni, hx, hy, hz);
+    }
+    if (p.coulomb_on)
+        adj_coulomb<T>(p, a, nu, s, t, lb, xi, ni, p.chg[lb][s], hx, hy, hz, gqs);
+}
+
+// One directed spring entry in a backward step: its Hessian term and its gradient sums.
+template <class NU>
+__device__ __forceinline__ void adj_spring(const AdjState &a, const NU nu, float cs, unsigned int c, float kk, float r0,
+                                           float4 xi, float4 li, float4 ni, float &hx, float &hy, float &hz, float &gk,
+                                           float &gr0)
+{
+    const int j = static_cast<int>(c & kSlotMask);
+    const float4 xj = a.x[j];
+    const float4 lj = a.xlo ? a.xlo[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 nj = (c & kEntryStatic) ? make_float4(0.f, 0.f, 0.f, 0.f) : nu[j];
+    float dx, dy, dz, d, inv, dv;
+    if (!spring_geometry(xi, xj, li, lj, r0, dx, dy, dz, d, inv, dv))
+        return;
+    const float ux = dx * inv, uy = dy * inv, uz = dz * inv;
+    hvp(cs * kk * dv, cs * kk, inv, ux, uy, uz, nj.x - ni.x, nj.y - ni.y, nj.z - ni.z, hx, hy, hz);
+    const float un = ux * ni.x + uy * ni.y + uz * ni.z;
+    gk += cs * dv * un;
+    gr0 -= cs * kk * un;
+}
+
+// lambda_x, lambda_v of a particle through one backward step; returns its new nu.
+__device__ __forceinline__ float4 adj_update(const Params &p, float m, float hx, float hy, float hz, float4 &lx, float4 &lv)
+{
+    const float b = m > 0.0f ? p.dt / m : 0.0f;
+    const float av = (m > 0.0f && p.visc_on) ? 1.0f - p.visc * p.dt / m : 1.0f;
+    const float mux = fmaf(p.dt, lx.x, lv.x), muy = fmaf(p.dt, lx.y, lv.y), muz = fmaf(p.dt, lx.z, lv.z);
+    const float nlx = lx.x + hx, nly = lx.y + hy, nlz = lx.z + hz;
+    const float nvx = av * mux, nvy = av * muy, nvz = av * muz;
+    lx = make_float4(nlx, nly, nlz, 0.f);
+    lv = make_float4(nvx, nvy, nvz, 0.f);
+    return make_float4(b * fmaf(p.dt, nlx, nvx), b * fmaf(p.dt, nly, nvy), b * fmaf(p.dt, nlz, nvz), 0.f);
 }
 
 // One backward step for every particle: reads nu of step n+1 and the positions at the start of
@@ -198,31 +249,13 @@ __global__ void __launch_bounds__(kStepBlock) k_adj_step(Params p, AdjState a)
                 const float gk = a.gk[sid], gr0 = a.gr0[sid];
                 if (c & kEntryInactive)
                     continue;
-                const int j = static_cast<int>(c & kSlotMask);
-                const float4 xj = a.x[j];
-                const float4 lj = a.xlo ? a.xlo[j] : make_float4(0.f, 0.f, 0.f, 0.f);
-                const float4 nj = (c & kEntryStatic) ? make_float4(0.f, 0.f, 0.f, 0.f) : a.nu_in[j];
-                float dx, dy, dz, d, inv, dv;
-                if (!spring_geometry(xi, xj, li, lj, r0, dx, dy, dz, d, inv, dv))
-                    continue;
-                const float ux = dx * inv, uy = dy * inv, uz = dz * inv;
-                hvp(cs * kk * dv, cs * kk, inv, ux, uy, uz, nj.x - ni.x, nj.y - ni.y, nj.z - ni.z, hx, hy, hz);
-                const float un = ux * ni.x + uy * ni.y + uz * ni.z;
-                a.gk[sid] = gk + cs * dv * un;
-                a.gr0[sid] = gr0 - cs * kk * un;
+                float nk = gk, nr0 = gr0;
+                adj_spring(a, PosConst{a.nu_in}, cs, c, kk, r0, xi, li, ni, hx, hy, hz, nk, nr0);
+                a.gk[sid] = nk;
+                a.gr0[sid] = nr0;
             }
         }
-        if (p.steric_on)
-        {
-            if (p.pl16)
-                adj_steric<T, 0>(p, a, s, t, xi, ni, hx, hy, hz);
-            else
-                adj_steric<T, 1>(p, a, s, t, xi, ni, hx, hy, hz);
-            if (p.pl[kListStericStatic].on && p.pl[kListStericStatic].cnt[s] > 0)
-                adj_steric<T, 2>(p, a, s, t, xi, ni, hx, hy, hz);
-        }
-        if (p.coulomb_on)
-            adj_coulomb<T>(p, a, s, t, lb, xi, ni, p.chg[lb][s], hx, hy, hz, gqs);
+        adj_nonbonded<T>(p, a, PosConst{a.nu_in}, s, t, lb, xi, ni, hx, hy, hz, gqs);
     }
     if (T > 1)
     {
@@ -241,16 +274,139 @@ __global__ void __launch_bounds__(kStepBlock) k_adj_step(Params p, AdjState a)
     }
     if (a.gq && p.coulomb_on)
         a.gq[p.perm[lb][s]] += gqs;
-    const float m = p.iprm[lb][s].x;
-    const float b = m > 0.0f ? p.dt / m : 0.0f;
-    const float av = (m > 0.0f && p.visc_on) ? 1.0f - p.visc * p.dt / m : 1.0f;
-    const float4 lx = a.lx[s], lv = a.lv[s];
-    const float mux = fmaf(p.dt, lx.x, lv.x), muy = fmaf(p.dt, lx.y, lv.y), muz = fmaf(p.dt, lx.z, lv.z);
-    const float nlx = lx.x + hx, nly = lx.y + hy, nlz = lx.z + hz;
-    const float nvx = av * mux, nvy = av * muy, nvz = av * muz;
-    a.lx[s] = make_float4(nlx, nly, nlz, 0.f);
-    a.lv[s] = make_float4(nvx, nvy, nvz, 0.f);
-    a.nu_out[s] = make_float4(b * fmaf(p.dt, nlx, nvx), b * fmaf(p.dt, nly, nvy), b * fmaf(p.dt, nlz, nvz), 0.f);
+    float4 lx = a.lx[s], lv = a.lv[s];
+    a.nu_out[s] = adj_update(p, p.iprm[lb][s].x, hx, hy, hz, lx, lv);
+    a.lx[s] = lx;
+    a.lv[s] = lv;
+}
+
+// `count` backward steps in one cooperative launch, from the last of an interval to its first (a.x and
+// a.xlo hold the positions of its first step, then of the next, npad apart), with a grid barrier
+// between two steps. What does not change over an interval stays in registers: the particle's lambda
+// and nu, the first kAdjHeld of its lane's spring entries and their gradient sums (a Calpha network has 19
+// entries a particle, so with 8 lanes none is left over); what is left over is read as k_adj_step reads it.
+// The sums run in k_adj_step's order. nu alternates between a.nu_in (at the start) and a.nu_out.
+// Bound: the partners' loads and the barrier. Measured (ncu, us a backward step): 10,000 particles 17.2 ->
+// 8.7, 1,999 with charge gradients 18.4 -> 8.7; training steps with the forward pass in k_run, which also
+// keeps the positions: 6,831 -> 4,822 us (10,000, 200 steps), 2,556 -> 1,909 us (1,999, 60 steps).
+constexpr int kAdjHeld = 3;
+// Two blocks of 320 an SM leave 102 registers a thread and hold 97,280 threads: 6,080 particles of 16 lanes,
+// 12,160 of 8; with 4 lanes (three blocks) 36,480.
+constexpr int kAdjRunBlock = 320;
+template <int T>
+__global__ void __launch_bounds__(kAdjRunBlock, T == 4 ? 3 : 2) k_adj_run(Params p, AdjState a, int count)
+{
+    const Ctl *ctl = p.ctl;
+    const int lb = ctl->lbuf;
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    const int s = g / T, t = g % T;
+    const bool lead = t == 0;
+    const bool active = s < p.n && !(p.flags[lb][s] & PF_STATIC);
+    const size_t stride = static_cast<size_t>(p.npad);
+    const float cs = p.k_spring_f * p.spring_scale;
+    const int deg = active && p.spring_on ? p.se_deg[s] : 0;
+    unsigned int col[kAdjHeld], sid[kAdjHeld];
+    float kk[kAdjHeld], r0[kAdjHeld], gk[kAdjHeld], gr0[kAdjHeld];
+#pragma unroll
+    for (int u = 0; u < kAdjHeld; ++u)
+    {
+        col[u] = kEntryInactive;
+        if (t + u * T < deg)
+        {
+            const size_t at = static_cast<size_t>(t + u * T) * stride + s;
+            col[u] = p.se_col[at];
+            kk[u] = p.se_k[at];
+            r0[u] = p.se_r0[at];
+            sid[u] = p.se_sid[at];
+            gk[u] = a.gk[sid[u]];
+            gr0[u] = a.gr0[sid[u]];
+        }
+    }
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 lx = zero, lv = zero, ni = zero;
+    float m = 0.0f, gq = 0.0f;
+    if (active)
+    {
+        ni = a.nu_in[s];
+        if (lead)
+        {
+            lx = a.lx[s];
+            lv = a.lv[s];
+            m = p.iprm[lb][s].x;
+            if (a.gq)
+                gq = a.gq[p.perm[lb][s]];
+        }
+    }
+    const float4 *first = a.x, *first_lo = a.xlo;
+    float4 *from = a.nu_in, *to = a.nu_out;
+    bool met = true;
+    for (int k = count - 1; k >= 0 && met; --k)
+    {
+        a.x = first + k * stride;
+        a.xlo = first_lo ? first_lo + k * stride : nullptr;
+        const PosShared nu{from};
+        float hx = 0.f, hy = 0.f, hz = 0.f, gqs = 0.f;
+        if (active)
+        {
+            const float4 xi = a.x[s], li = a.xlo ? a.xlo[s] : zero;
+#pragma unroll
+            for (int u = 0; u < kAdjHeld; ++u)
+                if (!(col[u] & kEntryInactive))
+                    adj_spring(a, nu, cs, col[u], kk[u], r0[u], xi, li, ni, hx, hy, hz, gk[u], gr0[u]);
+            for (int e = t + kAdjHeld * T; e < deg; e += T)
+            {
+                const size_t at = static_cast<size_t>(e) * stride + s;
+                const unsigned int c = p.se_col[at], id = p.se_sid[at];
+                if (!(c & kEntryInactive))
+                    adj_spring(a, nu, cs, c, p.se_k[at], p.se_r0[at], xi, li, ni, hx, hy, hz, a.gk[id], a.gr0[id]);
+            }
+            adj_nonbonded<T>(p, a, nu, s, t, lb, xi, ni, hx, hy, hz, gqs);
+        }
+        hx = group_sum<T>(hx);
+        hy = group_sum<T>(hy);
+        hz = group_sum<T>(hz);
+        if (a.gq)
+            gq += group_sum<T>(gqs);
+        if (lead && active)
+            ni = adj_update(p, m, hx, hy, hz, lx, lv);
+        if (lead && s < p.npad)
+            to[s] = ni; // zero for a particle that does not move
+        ni.x = __shfl_sync(0xffffffffu, ni.x, 0, T);
+        ni.y = __shfl_sync(0xffffffffu, ni.y, 0, T);
+        ni.z = __shfl_sync(0xffffffffu, ni.z, 0, T);
+        float4 *const now = to;
+        to = from;
+        from = now;
+        if (k > 0)
+            met = grid_barrier(p.order_sync, static_cast<unsigned int>(count - k), 0) != 0;
+    }
+    if (!met)
+    {
+        if (threadIdx.x == 0)
+            atomicOr(&p.ctl->status, ST_BARRIER);
+        return;
+    }
+#pragma unroll
+    for (int u = 0; u < kAdjHeld; ++u)
+        if (!(col[u] & kEntryInactive))
+        {
+            a.gk[sid[u]] = gk[u];
+            a.gr0[sid[u]] = gr0[u];
+        }
+    if (lead && active)
+    {
+        a.lx[s] = lx;
+        a.lv[s] = lv;
+        if (a.gq && p.coulomb_on)
+            a.gq[p.perm[lb][s]] = gq;
+    }
+    // the last block to finish: every block has left its last barrier
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(p.order_sync + 1, 1u) == gridDim.x - 1)
+    {
+        p.order_sync[0] = 0u;
+        p.order_sync[1] = 0u;
+    }
 }
 
 // Loss L = (1/n) sum_i |x_i - target_i|^2 at the current state (all particles), and the adjoint
@@ -401,6 +557,50 @@ int launch_adj_step(const Params &p, const AdjState &a, cudaStream_t st)
     else
         k_adj_step<4><<<nb, kStepBlock, 0, st>>>(p, a);
     return 1;
+}
+
+static const void *adj_run_fn(int lanes)
+{
+    return lanes == 16 ? reinterpret_cast<const void *>(&k_adj_run<16>)
+           : lanes == 8 ? reinterpret_cast<const void *>(&k_adj_run<8>)
+                        : reinterpret_cast<const void *>(&k_adj_run<4>);
+}
+
+static int adj_run_blocks(const Params &p, int lanes)
+{
+    return static_cast<int>((static_cast<long long>(p.npad) * lanes + kAdjRunBlock - 1) / kAdjRunBlock);
+}
+
+cudaError_t adj_run_lanes(const Params &p, int *lanes)
+{
+    *lanes = 0;
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess)
+        e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    for (int T = 16; T >= 4 && *lanes == 0 && e == cudaSuccess; T /= 2)
+    {
+        int per_sm = 0;
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, adj_run_fn(T), kAdjRunBlock, 0);
+        if (e == cudaSuccess && adj_run_blocks(p, T) <= per_sm * sms)
+            *lanes = T;
+    }
+    return e;
+}
+
+cudaError_t launch_adj_run(const Params &p, const AdjState &a, int count, int lanes, cudaStream_t st)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(adj_run_blocks(p, lanes)));
+    cfg.blockDim = dim3(kAdjRunBlock);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    void *args[] = {const_cast<Params *>(&p), const_cast<AdjState *>(&a), &count};
+    return cudaLaunchKernelExC(&cfg, adj_run_fn(lanes), args);
 }
 
 int launch_adj_init(const Params &p, const AdjState &a, const float4 *target, double *blk, unsigned int *done,

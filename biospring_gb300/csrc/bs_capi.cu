@@ -2236,6 +2236,26 @@ static int record_adjoint(bs_sim *s, int nsteps, int K, bool charges, bool keep_
     BS_CUDA(cudaMemsetAsync(s->adj_gr0, 0, sizeof(float) * 2 * std::max<size_t>(s->sp_i.size(), 1), s->stream));
     if (charges)
         BS_CUDA(cudaMemsetAsync(s->adj_gq, 0, sizeof(float) * s->n, s->stream));
+    // len steps from the current state, the positions each starts from to x (and remainders to lo; nullable)
+    auto forward = [&](int len, float4 *x, float4 *lo) {
+        if (p.run_on)
+            for (int k = 0; k < len; k += kRunMaxSteps)
+            {
+                const size_t at = static_cast<size_t>(k) * np;
+                launch_run(p, std::min(kRunMaxSteps, len - k), s->stream, x ? x + at : nullptr, lo ? lo + at : nullptr);
+                s->launches += 1;
+            }
+        else
+            for (int k = 0; k < len; ++k)
+            {
+                const size_t at = static_cast<size_t>(k) * np;
+                if (x)
+                    s->launches += launch_adj_save(p, x + at, lo ? lo + at : nullptr, s->stream);
+                s->launches += launch_step(p, MODE_STEP, s->stream);
+            }
+    };
+    int lanes = 0;
+    BS_CUDA(adj_run_lanes(p, &lanes));
     // forward: a checkpoint (caller order) and a rebuild at the start of every interval; the
     // positions of the last interval are kept as they are produced
     for (int seg = 0; seg < S; ++seg)
@@ -2245,15 +2265,9 @@ static int record_adjoint(bs_sim *s, int nsteps, int K, bool charges, bool keep_
         if (p.pos_lo[0])
             s->launches += launch_unsort(p, 3, s->adj_ck_lo + seg * n3, s->stream);
         s->launches += launch_rebuild(p, s->stream);
-        for (int k = 0; k < seg_len(seg); ++k)
-        {
-            if (keep_all || seg == S - 1)
-            {
-                const size_t at = (keep_all ? static_cast<size_t>(seg) * K + k : static_cast<size_t>(k)) * np;
-                s->launches += launch_adj_save(p, s->adj_seg + at, lo_seg ? lo_seg + at : nullptr, s->stream);
-            }
-            s->launches += launch_step(p, MODE_STEP, s->stream);
-        }
+        const bool keep = keep_all || seg == S - 1;
+        const size_t at = keep_all ? static_cast<size_t>(seg) * K * np : 0;
+        forward(seg_len(seg), keep ? s->adj_seg + at : nullptr, keep && lo_seg ? lo_seg + at : nullptr);
     }
     AdjState a{nullptr, nullptr, s->adj_lx, s->adj_lv, s->adj_nu[0], s->adj_nu[1], s->adj_gk, s->adj_gr0,
                charges ? s->adj_gq : nullptr};
@@ -2269,16 +2283,31 @@ static int record_adjoint(bs_sim *s, int nsteps, int K, bool charges, bool keep_
             s->launches += launch_set_positions(p, s->adj_ck_xyz + seg * n3, s->adj_ck_vel + seg * n3, s->stream,
                                                 p.pos_lo[0] ? s->adj_ck_lo + seg * n3 : nullptr);
             s->launches += launch_rebuild(p, s->stream);
-            for (int k = 0; !keep_all && k < len; ++k)
+            if (!keep_all)
             {
-                s->launches += launch_adj_save(p, s->adj_seg + k * np, lo_seg ? lo_seg + k * np : nullptr,
-                                               s->stream);
-                if (k < len - 1)
-                    s->launches += launch_step(p, MODE_STEP, s->stream);
+                // the positions of the interval's steps, the last of which need not be taken again
+                forward(len - 1, s->adj_seg, lo_seg);
+                const size_t at = static_cast<size_t>(len - 1) * np;
+                s->launches += launch_adj_save(p, s->adj_seg + at, lo_seg ? lo_seg + at : nullptr, s->stream);
             }
             s->launches += launch_adj_permute(p, a, s->adj_cx, s->adj_cv, 1, s->stream);
         }
-        for (int k = len - 1; k >= 0; --k)
+        if (lanes > 0)
+        {
+            const size_t at = keep_all ? static_cast<size_t>(seg) * K * np : 0;
+            for (int k1 = len, k0; k1 > 0; k1 = k0)
+            {
+                k0 = std::max(0, k1 - kRunMaxSteps);
+                a.x = s->adj_seg + at + k0 * np;
+                a.xlo = lo_seg ? lo_seg + at + k0 * np : nullptr;
+                a.nu_in = s->adj_nu[cur];
+                a.nu_out = s->adj_nu[cur ^ 1];
+                BS_CUDA(launch_adj_run(p, a, k1 - k0, lanes, s->stream));
+                s->launches += 1;
+                cur ^= (k1 - k0) & 1;
+            }
+        }
+        for (int k = len - 1; k >= 0 && lanes == 0; --k)
         {
             const size_t at = (keep_all ? static_cast<size_t>(seg) * K + k : static_cast<size_t>(k)) * np;
             a.x = s->adj_seg + at;

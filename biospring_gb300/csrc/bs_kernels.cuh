@@ -106,7 +106,9 @@ int launch_rigid(const Params &p, cudaStream_t stream);               // bs_rigi
 // count steps without a rebuild in between: one kernel where the system allows (Params::run_on)
 int launch_steps(const Params &p, int count, cudaStream_t stream);
 // bs_run.cu: the kernel of several steps, its blocks, and whether they are resident at once
-cudaError_t launch_run(const Params &p, int count, cudaStream_t stream);
+// (save, save_lo, nullable: the positions every step starts from and their remainders, npad a step)
+cudaError_t launch_run(const Params &p, int count, cudaStream_t stream, float4 *save = nullptr,
+                       float4 *save_lo = nullptr);
 cudaError_t run_fits(const Params &p, bool *fits);
 int run_blocks(const Params &p);
 // Steps of one launch (10 in the default schedule) and the polls after which a barrier gives up (some
@@ -145,6 +147,10 @@ struct AdjState
     float *gq;       // dL/dq per caller id (null: no charge gradients)
 };
 int launch_adj_step(const Params &p, const AdjState &a, cudaStream_t stream);
+// count backward steps in one kernel with `lanes` lanes a particle, the most (of 16, 8, 4) whose grid is
+// resident at once (0: none is)
+cudaError_t adj_run_lanes(const Params &p, int *lanes);
+cudaError_t launch_adj_run(const Params &p, const AdjState &a, int count, int lanes, cudaStream_t stream);
 int launch_adj_init(const Params &p, const AdjState &a, const float4 *target, double *blk, unsigned int *done,
                     double *loss, cudaStream_t stream);
 int launch_adj_permute(const Params &p, const AdjState &a, float4 *cx, float4 *cv, int dir, cudaStream_t stream);

@@ -68,7 +68,7 @@ __device__ __forceinline__ void probe_step(const Params &p, const float *part, f
 }
 
 template <int SM, int T, bool LEAN>
-__global__ void __launch_bounds__(kStepKernelBlock, kStepMinBlocks) k_run(Params p, int count)
+__global__ void __launch_bounds__(kStepKernelBlock, kStepMinBlocks) k_run(Params p, int count, float4 *save, float4 *save_lo)
 {
     Ctl *ctl = p.ctl;
     if (status_of(ctl) != 0)
@@ -98,6 +98,13 @@ __global__ void __launch_bounds__(kStepKernelBlock, kStepMinBlocks) k_run(Params
         for (int q = 0; q < 6; ++q)
             e[q] = 0.0f;
         const int sb = sb0 ^ (k & 1);
+        if (save && g % T == 0 && g / T < p.n)
+        {
+            const size_t at = static_cast<size_t>(k) * p.npad + g / T;
+            save[at] = p.pos[sb][g / T];
+            if (!LEAN && save_lo)
+                save_lo[at] = p.pos_lo[sb][g / T];
+        }
         int pend = particle_step<MODE_STEP, SM, T, true, LEAN, PosShared>(p, g / T, g % T, p.n, sb, lb, ext && k == 0,
                                                                           prb, e);
         float *part = p.run_probe + static_cast<size_t>(k & 1) * 8 * gridDim.x; // read until the next step's barrier
@@ -217,7 +224,7 @@ cudaError_t run_fits(const Params &p, bool *fits)
     return e;
 }
 
-cudaError_t launch_run(const Params &p, int count, cudaStream_t st)
+cudaError_t launch_run(const Params &p, int count, cudaStream_t st, float4 *save, float4 *save_lo)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(run_blocks(p)));
@@ -228,7 +235,7 @@ cudaError_t launch_run(const Params &p, int count, cudaStream_t st)
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    void *args[] = {const_cast<Params *>(&p), &count};
+    void *args[] = {const_cast<Params *>(&p), &count, &save, &save_lo};
     return cudaLaunchKernelExC(&cfg, run_kernel(p), args);
 }
 
