@@ -535,23 +535,25 @@ __device__ __forceinline__ float lj_pair(float r2, bool ok, float pw, float fhi_
 {
     const float inv2 = recip_lj(r2);
     const float i6 = inv2 * inv2 * inv2;
-    const float t6 = pw * pj.w * i6;
+    // the products are rounded before the differences in every build, so that a step whose energy is not
+    // summed gives the same force bits (without it the compiler may fuse a product it uses once)
+    const float t6 = __fmul_rn(pw * pj.w, i6);
     float fod, de;
     if (SM == BS_STERIC_LJ_12_6_AMBER)
     {
-        const float t12 = fhi_i * hj * i6 * i6;
+        const float t12 = __fmul_rn(fhi_i * hj * i6, i6);
         de = t12 - 2.0f * t6;
         fod = 12.0f * (t6 - t12) * inv2;
     }
     else if (SM == BS_STERIC_LJ_8_6_LEWITT)
     {
-        const float t8 = fhi_i * hj * i6 * inv2;
+        const float t8 = __fmul_rn(fhi_i * hj * i6, inv2);
         de = 3.0f * t8 - 4.0f * t6;
         fod = 24.0f * (t6 - t8) * inv2;
     }
     else
     {
-        const float t8 = fhi_i * hj * i6 * inv2;
+        const float t8 = __fmul_rn(fhi_i * hj * i6, inv2);
         de = t8 - t6;
         fod = (6.0f * t6 - 8.0f * t8) * inv2;
     }
@@ -1157,6 +1159,7 @@ __device__ __forceinline__ int particle_step(const Params &p, const int s, const
             e[3] = es * p.k_hydro_e * p.hydro_scale;
         }
     }
+    constexpr bool kEnergy = MODE != MODE_STEP_PART;
     if (T > 1)
     {
         // every lane of the warp takes part in the group reductions
@@ -1164,7 +1167,7 @@ __device__ __forceinline__ int particle_step(const Params &p, const int s, const
         fy = group_sum<T>(fy);
         fz = group_sum<T>(fz);
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
+        for (int k = 0; k < 4 && kEnergy; ++k)
             e[k] = group_sum<T>(e[k]);
         if (!lead)
         {
@@ -1192,7 +1195,8 @@ __device__ __forceinline__ int particle_step(const Params &p, const int s, const
             cx = group_sum<32>(cx);
             cy = group_sum<32>(cy);
             cz = group_sum<32>(cz);
-            ce = group_sum<32>(ce);
+            if (kEnergy)
+                ce = group_sum<32>(ce);
             if (lane == src)
             {
                 fx = fmaf(cx, p.k_elec_f, fx);
@@ -1206,7 +1210,7 @@ __device__ __forceinline__ int particle_step(const Params &p, const int s, const
     {
         if (!active)
         {
-            if (MODE == MODE_STEP)
+            if (MODE != MODE_FORCES)
             {
                 p.pos[sb ^ 1][s] = pi;
                 p.vel[sb ^ 1][s] = p.vel[sb][s];
@@ -1257,7 +1261,7 @@ __device__ __forceinline__ int particle_step(const Params &p, const int s, const
                 fx += ex;
                 fy += ey;
                 fz += ez;
-                if (MODE == MODE_STEP && (ex != 0.f || ey != 0.f || ez != 0.f))
+                if (MODE != MODE_FORCES && (ex != 0.f || ey != 0.f || ez != 0.f))
                 {
                     xf[0] = 0.f;
                     xf[1] = 0.f;
@@ -1330,9 +1334,10 @@ __device__ __forceinline__ int particle_step(const Params &p, const int s, const
             }
         }
     }
+    if (kEnergy)
 #pragma unroll
-    for (int k = 0; k < 6; ++k)
-        eacc[k] += e[k];
+        for (int k = 0; k < 6; ++k)
+            eacc[k] += e[k];
     return pend;
 }
 

@@ -94,6 +94,9 @@ enum StepMode
 {
     MODE_STEP = 0,   // forces + Euler step (SpringNetwork::computeStep)
     MODE_FORCES = 1, // forces and energies only (SpringNetwork::computeForces)
+    // A step with further steps enqueued behind it in the same call: every way to read energies completes
+    // those first (or fails), so this step's could not be seen and are not summed.
+    MODE_STEP_PART = 2,
 };
 
 // Launchers (all asynchronous on `stream`); each returns the number of kernels launched.
