@@ -72,21 +72,8 @@ constexpr int kGatherU = 4;
 #ifndef BS_GRID_DIV
 #define BS_GRID_DIV 2
 #endif
-// the cell-block list build walks the bounded runs as one packed sequence when there are many
-#ifndef BS_PL_PACK
-#define BS_PL_PACK (BS_GRID_DIV > 1)
-#endif
-#ifndef BS_PL_WARPS
-#define BS_PL_WARPS 8
-#endif
-#ifndef BS_PL_STAGE
-#define BS_PL_STAGE 2048
-#endif
 constexpr int kGridDiv = BS_GRID_DIV; // cell-block list build: cells per list radius (stencil of +-kGridDiv cells)
 constexpr int kSparseDiv = 1;         // warp-per-particle list build (sparse systems, batches): cells of the radius
-constexpr int kPlWarps = BS_PL_WARPS; // warps per block (one cell) in the pair-list build
-constexpr int kPlStage = BS_PL_STAGE; // candidate positions staged in shared memory per block
-constexpr int kPlMinBlocks = 4;       // resident list-build blocks per SM (the stage allows 4)
 constexpr int kPlBatch = 16;         // home particles per warp
 constexpr int kPlBatchesPerCell = 4; // warps per cell (a cell with more than 64 particles loops)
 
@@ -103,6 +90,7 @@ enum StepMode
 int launch_rebuild(const Params &p, cudaStream_t stream);
 cudaError_t launch_order(const Params &p, cudaStream_t stream); // bs_order.cu
 cudaError_t order_blocks(const Params &p, int *blocks);
+int launch_pairlist(const Params &p, cudaStream_t stream); // bs_list.cu
 int launch_step(const Params &p, int mode, cudaStream_t stream);      // step kernel, then the bodies
 int launch_step_only(const Params &p, int mode, cudaStream_t stream); // the step kernel alone
 int launch_rigid(const Params &p, cudaStream_t stream);               // bs_rigid.cu
