@@ -17,6 +17,7 @@ constexpr int kStepBlock = 128; // adjoint and diagnostic kernels
 // (1024 resident threads: at most 64 registers)
 constexpr int kStepKernelBlock = BS_STEP_BLOCK;
 constexpr int kStepMinBlocks = BS_STEP_MIN_BLOCKS;
+constexpr int kStepPartBlock = 128; // of the steps whose energies are not summed
 constexpr int kBuildBlock = 128;
 constexpr int kBuildLanes = 8;    // threads per slot of the spring-table rebuild when the table fits L2
 // k_order: most blocks of its grid, and the threads a particle it is sized for (small systems use as few
