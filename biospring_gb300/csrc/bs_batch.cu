@@ -9,19 +9,18 @@
 // Rebuild: k_order (bs_order.cu), then k_batch_pairlist (one warp per home particle: systems are
 // sparse, a cell holds a few particles).
 //
-// Step: k_batch_run, a persistent kernel launched with thread-block clusters. A cluster owns a
-// list of whole systems (a host-side longest-processing-time assignment) and runs each of them
-// for the period's steps before moving to the next, with one cluster barrier per step; no other
-// synchronisation is needed because systems are independent. A system's state stays in L2
-// (and L1) across its steps. The per-particle work is the single-system routine
-// (particle_step), so a system follows the same arithmetic as when it is stepped alone.
+// Step: k_batch_run, a persistent kernel, launched cooperatively. Its blocks form groups; a group owns
+// a list of whole systems (a host-side longest-processing-time assignment) and runs each of them for the
+// period's steps before moving to the next, with one barrier of the group per step; no other
+// synchronisation is needed because systems are independent. A group has blocks in proportion to its
+// systems' work, so that an ensemble of unequal systems ends together. A system's state stays in L2
+// (and L1) across its steps. The per-particle work is the single-system routine (particle_step), so a
+// system follows the same arithmetic as when it is stepped alone.
 //
 // Lists go stale per system: a step whose end positions drift more than half the list skin
 // records its index in stale_at[b]; the system stops after that step and resumes after the next
 // rebuild. At the end of a launch every system's state is put in the buffer the launch's nominal
 // step count implies, so the next rebuild sees one consistent buffer index.
-
-#include <cooperative_groups.h>
 
 #include "bs_device.cuh"
 
@@ -29,8 +28,6 @@ namespace bsg
 {
 namespace
 {
-
-namespace cg = cooperative_groups;
 
 // the batched list build loads a warp's next home while it lists the current one
 #ifndef BS_BPL_PREFETCH
@@ -335,36 +332,47 @@ __device__ __forceinline__ void block_energy_partial(const float (&e)[NE], float
 template <int SM, int T, bool LEAN>
 __global__ void __launch_bounds__(kBatchMaxBlock, 2) k_batch_run(Params p, int chunk)
 {
-    cg::cluster_group cl = cg::this_cluster();
-    const int rank = static_cast<int>(cl.block_rank());
-    const int csize = static_cast<int>(cl.num_blocks());
-    const int cid = static_cast<int>(blockIdx.x) / csize;
     Ctl *ctl = p.ctl;
     if (status_of(ctl) & kRebuildBlocking)
         return; // uniform: the status does not change while this kernel runs
+    const int cid = p.blk_group[blockIdx.x];
+    const int rank = static_cast<int>(blockIdx.x) - p.grp_start[cid];
+    const int csize = p.grp_start[cid + 1] - p.grp_start[cid];
+    unsigned int gen = 0;
+    // all blocks of the group; true if a thread came with pend set. A barrier that gives up (its wait is
+    // bounded) ends the launch as failed. A flag raised at one meeting is cleared by rank 0 between the
+    // next two: the meeting after a raised flag and the first of the next system carry none.
+    bool failed = false, raised = false;
+    auto meet = [&](int pend) -> bool {
+        if (csize == 1)
+            return __syncthreads_or(pend) != 0;
+        const int r = group_barrier(p.grp_arrive + cid, static_cast<unsigned int>(csize), ++gen, pend);
+        if (raised && rank == 0 && threadIdx.x == 0)
+            atomicAnd(p.grp_arrive + cid, ~(1u << (30 + ((gen - 1u) & 1u))));
+        raised = r == 2;
+        failed = failed || r == 0;
+        return r != 1;
+    };
     const int sb0 = ctl->sbuf, lb = ctl->lbuf;
     const long long upto = ctl->nominal + chunk;
     const int out_parity = chunk & 1;
     const int stride = csize * static_cast<int>(blockDim.x);
     const int me = rank * static_cast<int>(blockDim.x) + static_cast<int>(threadIdx.x);
-    for (int q = p.cl_start[cid]; q < p.cl_start[cid + 1]; ++q)
+    for (int q = p.cl_start[cid]; q < p.cl_start[cid + 1] && !failed; ++q)
     {
         const int b = p.cl_sys[q];
         const int n0 = p.sys_start[b], n1 = p.sys_start[b + 1];
         const long long done = p.sys_steps[b];
-        const bool dead = (p.sys_status[b] & ST_NONFINITE) != 0;
         // stale_at[b] < done: the list went stale before this launch (no rebuild since)
-        long long stale = p.stale_at[b];
-        // every thread of the cluster has read this system's control words before any of them
+        const bool dead = (p.sys_status[b] & ST_NONFINITE) != 0 || p.stale_at[b] < done;
+        // every thread of the group has read this system's control words before any of them
         // can write them (a step records staleness and non-finite positions)
-        cl.sync();
+        meet(0);
         int k = 0;
         float e[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         const int span = (n1 - n0) * T;
-        // Loop condition: every thread of the cluster evaluates the same values, because a step
-        // only records its own index in stale_at, which is >= done + k for steps not yet waited
-        // for at the barrier.
-        while (!dead && stale >= done + k && done + k < upto)
+        bool stop = dead; // the same in every thread of the group
+        while (!stop && !failed && done + k < upto)
         {
             const int sb = sb0 ^ (k & 1);
 #pragma unroll
@@ -384,12 +392,13 @@ __global__ void __launch_bounds__(kBatchMaxBlock, 2) k_batch_run(Params p, int c
                     atomicOr(&p.sys_status[b], ST_NONFINITE);
             }
             ++k;
-            cl.sync();
-            stale = atomicAdd(reinterpret_cast<unsigned long long *>(&p.stale_at[b]), 0ull);
+            stop = meet(pend);
         }
+        if (failed)
+            break;
         if (k == 0)
             continue;
-        float *part = p.sys_part + (static_cast<size_t>(b) * kMaxCluster + rank) * 16;
+        float *part = p.sys_part + static_cast<size_t>(blockIdx.x) * 16;
         block_energy_partial<6>(e, part);
         if ((k & 1) != out_parity)
         {
@@ -403,13 +412,13 @@ __global__ void __launch_bounds__(kBatchMaxBlock, 2) k_batch_run(Params p, int c
                     p.pos_lo[to][s] = p.pos_lo[from][s];
             }
         }
-        cl.sync();
+        meet(0);
         if (rank == 0 && threadIdx.x < 6)
         {
             float hi = 0.0f, lo = 0.0f;
             for (int r = 0; r < csize; ++r)
             {
-                const float *pr = p.sys_part + (static_cast<size_t>(b) * kMaxCluster + r) * 16;
+                const float *pr = part + static_cast<size_t>(r) * 16;
                 ff_add(hi, lo, __ldcg(pr + 2 * threadIdx.x), __ldcg(pr + 2 * threadIdx.x + 1));
             }
             // e[] order: spring, steric, Coulomb, hydrophobic, IMPALA, kinetic
@@ -419,6 +428,15 @@ __global__ void __launch_bounds__(kBatchMaxBlock, 2) k_batch_run(Params p, int c
         }
         if (rank == 0 && threadIdx.x == 0)
             p.sys_steps[b] = done + k;
+    }
+    if (failed && threadIdx.x == 0)
+        atomicOr(&ctl->status_pending, ST_BARRIER);
+    // the last block of the group to finish: every block has left its last barrier
+    __syncthreads();
+    if (threadIdx.x == 0 && csize > 1 && atomicAdd(p.grp_arrive + p.ncl + cid, 1u) == static_cast<unsigned int>(csize - 1))
+    {
+        p.grp_arrive[cid] = 0u;
+        p.grp_arrive[p.ncl + cid] = 0u;
     }
 }
 
@@ -462,8 +480,9 @@ __global__ void __launch_bounds__(256) k_batch_finish(Params p, int chunk)
         ctl->sbuf ^= chunk & 1;
         ctl->lagging = sh_lag;
         ctl->dead = sh_dead;
-        if (sh_dead)
-            atomicOr(&ctl->status, ST_NONFINITE);
+        const int bits = (sh_dead ? ST_NONFINITE : 0) | atomicExch(&ctl->status_pending, 0);
+        if (bits)
+            atomicOr(&ctl->status, bits);
     }
 }
 
@@ -532,15 +551,13 @@ cudaError_t launch_batch_run(const Params &p, const BatchShape &shape, int chunk
     if (!fn)
         return cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(p.ncl * shape.cluster), 1, 1);
+    cfg.gridDim = dim3(static_cast<unsigned>(p.nblk), 1, 1);
     cfg.blockDim = dim3(static_cast<unsigned>(shape.block), 1, 1);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = static_cast<unsigned>(shape.cluster);
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     void *args[] = {const_cast<Params *>(&p), &chunk};
@@ -553,22 +570,20 @@ int launch_batch_finish(const Params &p, int chunk, cudaStream_t st)
     return 1;
 }
 
-cudaError_t batch_max_clusters(const Params &p, const BatchShape &shape, int *out)
+cudaError_t batch_max_blocks(const Params &p, const BatchShape &shape, int *out)
 {
+    *out = 0;
     const void *fn = batch_run_kernel(p.steric_mode, shape.lanes, BS_LEAN && !p.hydro_on && !p.pos_lo[0]);
     if (!fn)
         return cudaErrorInvalidValue;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(shape.cluster), 1, 1);
-    cfg.blockDim = dim3(static_cast<unsigned>(shape.block), 1, 1);
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = static_cast<unsigned>(shape.cluster);
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaOccupancyMaxActiveClusters(out, fn, &cfg);
+    int dev = 0, sms = 0, per_sm = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess)
+        e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, shape.block, 0);
+    *out = per_sm * sms;
+    return e;
 }
 
 } // namespace bsg

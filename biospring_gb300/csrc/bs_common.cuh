@@ -241,9 +241,13 @@ struct Params
     long long *sys_steps;     // [nsys] steps completed by each system
     long long *stale_at;      // [nsys] first step whose end positions left the list skin
     double *sys_energy;       // [nsys * 8] BS_ENERGY_* of each system's last step
-    float *sys_part;          // [nsys * kMaxCluster * 16] per-block energy partials (hi, lo)
-    const int *cl_start;      // [ncl + 1] systems of each cluster of the persistent kernel
+    float *sys_part;          // [kBatchMaxBlocks * 16] energy partials (hi, lo) of each block's current system
+    const int *cl_start;      // [ncl + 1] systems of each block group of the persistent kernel
     const int *cl_sys;        // [nsys]
+    const int *grp_start;     // [ncl + 1] blocks of each group
+    const int *blk_group;     // [nblk] group of each block
+    unsigned int *grp_arrive; // [2 ncl] barrier words, then counts of finished blocks, 0 between launches
+    int nblk;
     int ncl;
     // rigid bodies (nbody = 0: none)
     int nbody;
@@ -275,8 +279,6 @@ struct Params
     float *frame_xyz;               // [frame_cap][3n], device view of the host ring
     FrameHeader *frame_hdr;         // [frame_cap]
 };
-
-constexpr int kMaxCluster = 16;
 
 // Systems without nonbonded terms: particles per cell the host aims at, and the cells a system of
 // n particles may have. A particle is ranked within its cell by counting (k_order), so the sort's time goes

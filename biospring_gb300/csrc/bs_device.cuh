@@ -173,19 +173,19 @@ __device__ __forceinline__ bool pair_in(float r2, float lo2, float hi2, float4 p
     return exact_pair_test(pi, pj, cutoff, nonzero);
 }
 
-// All blocks of the (cooperative) grid meet; gen counts the meetings of this launch from 1. Returns 1,
+// `blocks` blocks of a cooperative grid meet; gen counts their meetings of this launch from 1. Returns 1,
 // or 2 in every block alike if a thread of any block came with `pend` set, or 0 if this block gave the
 // (bounded) wait up: the others then do so too, and the launch ends without advancing the state.
 // Two flag bits, by the parity of gen: a block may already be at the next meeting when another reads
 // the word, but never two ahead.
 constexpr unsigned int kRunCount = (1u << 30) - 1u;
-__device__ __forceinline__ int grid_barrier(unsigned int *arrive, unsigned int gen, int pend)
+__device__ __forceinline__ int group_barrier(unsigned int *arrive, unsigned int blocks, unsigned int gen, int pend)
 {
     __shared__ int met;
     const int any = __syncthreads_or(pend);
     if (threadIdx.x == 0)
     {
-        const unsigned int want = gen * gridDim.x, flag = 1u << (30 + (gen & 1u));
+        const unsigned int want = gen * blocks, flag = 1u << (30 + (gen & 1u));
         if (any)
             atomicOr(arrive, flag);
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrive) : "memory");
@@ -198,6 +198,11 @@ __device__ __forceinline__ int grid_barrier(unsigned int *arrive, unsigned int g
     }
     __syncthreads();
     return met;
+}
+
+__device__ __forceinline__ int grid_barrier(unsigned int *arrive, unsigned int gen, int pend)
+{
+    return group_barrier(arrive, gridDim.x, gen, pend);
 }
 
 // Knuth's TwoSum: s = fl(a + b) and s + err == a + b exactly (round-to-nearest, no contraction).

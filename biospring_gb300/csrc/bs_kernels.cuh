@@ -155,11 +155,12 @@ struct BatchShape
 {
     int block;   // threads per block
     int lanes;   // threads per particle (1, 2, 4, 8)
-    int cluster; // blocks per cluster (1, 2, 4, 8)
+    int cluster; // mean blocks per group (1, 2, 4, 8)
 };
 int launch_batch_pairlist(const Params &p, cudaStream_t stream);
 cudaError_t launch_batch_run(const Params &p, const BatchShape &shape, int chunk, cudaStream_t stream);
 int launch_batch_finish(const Params &p, int chunk, cudaStream_t stream);
-cudaError_t batch_max_clusters(const Params &p, const BatchShape &shape, int *out);
+cudaError_t batch_max_blocks(const Params &p, const BatchShape &shape, int *out); // resident at once
+constexpr int kBatchMaxBlocks = 4096; // of a launch
 
 } // namespace bsg

@@ -380,7 +380,7 @@ int bs_adjoint(bs_sim *sim, int32_t nsteps, int32_t checkpoint, const float *tar
  * a spring may not join two systems), then declare the partition before bs_setup:
  * system b owns particles [offsets[b], offsets[b+1]). All systems share one bs_config.
  * bs_step advances every system by nsteps with a persistent kernel in which a
- * thread-block cluster owns whole systems; bs_get_positions / bs_get_velocities /
+ * group of thread blocks owns whole systems; bs_get_positions / bs_get_velocities /
  * bs_compute_forces work on the concatenation, bs_get_energies gives the sums over systems and
  * bs_get_system_energies each system's. External forces and the pair/cell diagnostics are for
  * single systems (BS_E_STATE); rigid bodies, the probe and field grids are BS_E_ARG at bs_setup. */
@@ -390,7 +390,8 @@ int bs_set_systems(bs_sim *sim, int32_t nsys, const int64_t *offsets);
 int bs_get_system_energies(bs_sim *sim, double *out);
 
 /* Launch shape of the persistent batched step kernel: threads per block (128, 256, 512),
- * threads per particle (1, 2, 4, 8) and blocks per cluster (1, 2, 4, 8). */
+ * threads per particle (1, 2, 4, 8) and mean number of blocks (1, 2, 4, 8) of the groups that own
+ * whole systems; a group has blocks in proportion to its systems' work. */
 int bs_set_batch_shape(bs_sim *sim, int32_t block, int32_t lanes, int32_t cluster);
 int bs_get_batch_shape(bs_sim *sim, int32_t shape[3]);
 
