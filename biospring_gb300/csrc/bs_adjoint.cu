@@ -412,7 +412,7 @@ __global__ void __launch_bounds__(kAdjRunBlock, T == 4 ? 3 : 2) k_adj_run(Params
 // Loss L = (1/n) sum_i |x_i - target_i|^2 at the current state (all particles), and the adjoint
 // state at the final step: lambda_x = 2 (x - target) / n, lambda_v = 0, nu = b dt lambda_x
 // (zero for static particles). Per-block partial sums in FP64; the last block writes the total.
-__global__ void __launch_bounds__(256) k_adj_init(Params p, AdjState a, const float4 *target, double *blk,
+__global__ void __launch_bounds__(256) k_adj_init(Params p, AdjState a, const float *target, double *blk,
                                                   unsigned int *done, double *loss)
 {
     const Ctl *ctl = p.ctl;
@@ -425,8 +425,9 @@ __global__ void __launch_bounds__(256) k_adj_init(Params p, AdjState a, const fl
         if (s < p.n)
         {
             const int id = p.perm[lb][s];
-            const float4 x = p.pos[sb][s], tg = target[id];
-            float dx = x.x - tg.x, dy = x.y - tg.y, dz = x.z - tg.z;
+            const float4 x = p.pos[sb][s];
+            const float *tg = target + 3 * static_cast<size_t>(id);
+            float dx = x.x - tg[0], dy = x.y - tg[1], dz = x.z - tg[2];
             if (p.pos_lo[0])
             {
                 const float4 lo = p.pos_lo[sb][s];
@@ -603,7 +604,7 @@ cudaError_t launch_adj_run(const Params &p, const AdjState &a, int count, int la
     return cudaLaunchKernelExC(&cfg, adj_run_fn(lanes), args);
 }
 
-int launch_adj_init(const Params &p, const AdjState &a, const float4 *target, double *blk, unsigned int *done,
+int launch_adj_init(const Params &p, const AdjState &a, const float *target, double *blk, unsigned int *done,
                     double *loss, cudaStream_t st)
 {
     k_adj_init<<<(p.npad + 255) / 256, 256, 0, st>>>(p, a, target, blk, done, loss);

@@ -23,6 +23,10 @@ namespace
 
 thread_local std::string g_last_error;
 
+// Largest result a kernel writes straight into page-locked host memory; beyond, a copy engine's transfer
+// of the whole array is the faster way out.
+constexpr size_t kDirectOut = 256 * 1024;
+
 struct DeviceBuffers
 {
     std::vector<void *> owned;
@@ -81,7 +85,10 @@ struct bs_sim
     Params p{};
     Ctl *ctl_host = nullptr; // pinned mirror
     float *staging = nullptr; // device float[3n]
-    float *ext_stage = nullptr; // pinned float[3n]: external forces from pageable caller memory
+    // pinned float[3n]: the caller's pageable arrays on their way in and (small systems) out; stage_event
+    // marks the last copy out of it still in flight
+    float *stage_h = nullptr;
+    cudaEvent_t stage_event = nullptr;
     int *one_host = nullptr;    // pinned constant 1 (source of the ext_pending flag)
     long long ctl_read_at = -1; // launch count when ctl_host was last read (all work finished)
     int step_blocks = 0;
@@ -104,13 +111,14 @@ struct bs_sim
     int *grp_start_d = nullptr, *blk_group_d = nullptr;
     // adjoint: directed spring ids of the caller-order CSR, scratch, and the captured run
     std::vector<unsigned int> csr_sid;
-    std::vector<int> csr_pos; // CSR position of each spring's two directed entries
     unsigned int *sp_sid_d = nullptr;
+    float *sp_stage_d = nullptr; // float[2 ns]: new spring parameters, caller order
     DeviceBuffers adj_dev;
     int adj_ck_cap = 0, adj_seg_cap = 0;
     float *adj_ck_xyz = nullptr, *adj_ck_vel = nullptr, *adj_ck_lo = nullptr;
     float4 *adj_seg = nullptr, *adj_seg_lo = nullptr, *adj_lx = nullptr, *adj_lv = nullptr, *adj_nu[2] = {nullptr, nullptr};
-    float4 *adj_cx = nullptr, *adj_cv = nullptr, *adj_target = nullptr;
+    float4 *adj_cx = nullptr, *adj_cv = nullptr;
+    float *adj_target = nullptr; // [3n], caller order
     float *adj_gk = nullptr, *adj_gr0 = nullptr, *adj_ok = nullptr, *adj_or0 = nullptr;
     double *adj_blk = nullptr, *adj_loss = nullptr;
     unsigned int *adj_done = nullptr;
@@ -193,6 +201,7 @@ void release_device(bs_sim *s)
     s->adj_ck_cap = 0;
     s->adj_seg_cap = 0;
     s->sp_sid_d = nullptr;
+    s->sp_stage_d = nullptr;
     s->diag_out = nullptr;
     s->diag_count = nullptr;
     s->diag_cap = 0;
@@ -205,10 +214,15 @@ void release_device(bs_sim *s)
         cudaFreeHost(s->ctl_host);
         s->ctl_host = nullptr;
     }
-    if (s->ext_stage)
+    if (s->stage_h)
     {
-        cudaFreeHost(s->ext_stage);
-        s->ext_stage = nullptr;
+        cudaFreeHost(s->stage_h);
+        s->stage_h = nullptr;
+    }
+    if (s->stage_event)
+    {
+        cudaEventDestroy(s->stage_event);
+        s->stage_event = nullptr;
     }
     if (s->one_host)
     {
@@ -232,6 +246,32 @@ int read_ctl(bs_sim *s)
     BS_CUDA(cudaMemcpyAsync(s->ctl_host, s->p.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s->stream));
     BS_CUDA(cudaStreamSynchronize(s->stream));
     s->ctl_read_at = s->launches;
+    return BS_OK;
+}
+
+// Kind of memory a caller's pointer is (cudaMemoryTypeUnregistered: pageable host memory).
+cudaMemoryType memory_type(const void *p)
+{
+    cudaPointerAttributes attr{};
+    if (cudaPointerGetAttributes(&attr, p) == cudaSuccess)
+        return attr.type;
+    cudaGetLastError(); // clear the query's error
+    return cudaMemoryTypeUnregistered;
+}
+
+// Enqueues a copy of up to 3n floats of the caller's to the device. A pageable source goes through the
+// handle's pinned buffer, so the caller may reuse it when this returns and the call waits for nothing but an
+// earlier copy out of that buffer; any other must stay unchanged until the stream is waited for.
+int upload(bs_sim *s, float *dst, const float *src, size_t floats, bool pinned)
+{
+    if (!pinned)
+    {
+        BS_CUDA(cudaEventSynchronize(s->stage_event));
+        std::memcpy(s->stage_h, src, floats * sizeof(float));
+    }
+    BS_CUDA(cudaMemcpyAsync(dst, pinned ? src : s->stage_h, floats * sizeof(float), cudaMemcpyHostToDevice, s->stream));
+    if (!pinned)
+        BS_CUDA(cudaEventRecord(s->stage_event, s->stream));
     return BS_OK;
 }
 
@@ -1054,7 +1094,6 @@ int bs_setup(bs_sim *s, const bs_config *cfg)
     std::vector<float> kk(std::max(nnz, 1)), rr(std::max(nnz, 1));
     std::vector<int> fillp(row.begin(), row.end() - 1);
     s->csr_sid.assign(std::max(nnz, 1), 0u);
-    s->csr_pos.assign(2 * s->sp_i.size(), 0);
     auto partner_code = [&](int a, int b) {
         uint32_t code = static_cast<uint32_t>(b);
         if (s->is_static[b])
@@ -1071,13 +1110,11 @@ int bs_setup(bs_sim *s, const bs_config *cfg)
         kk[e] = s->sp_k[t];
         rr[e] = s->sp_r0[t];
         s->csr_sid[e] = static_cast<unsigned int>(2 * t);
-        s->csr_pos[2 * t] = e;
         e = fillp[b]++;
         col[e] = partner_code(b, a);
         kk[e] = s->sp_k[t];
         rr[e] = s->sp_r0[t];
         s->csr_sid[e] = static_cast<unsigned int>(2 * t + 1);
-        s->csr_pos[2 * t + 1] = e;
     }
     int maxdeg = 1;
     for (int64_t i = 0; i < n; ++i)
@@ -1194,7 +1231,8 @@ int bs_setup(bs_sim *s, const bs_config *cfg)
     BS_CUDA(s->dev.alloc(&p.ctl, 1));
     BS_CUDA(s->dev.alloc(&s->staging, 3 * static_cast<size_t>(n)));
     BS_CUDA(cudaMallocHost(reinterpret_cast<void **>(&s->ctl_host), sizeof(Ctl)));
-    BS_CUDA(cudaMallocHost(reinterpret_cast<void **>(&s->ext_stage), sizeof(float) * 3 * n));
+    BS_CUDA(cudaMallocHost(reinterpret_cast<void **>(&s->stage_h), sizeof(float) * 3 * n));
+    BS_CUDA(cudaEventCreateWithFlags(&s->stage_event, cudaEventDisableTiming));
     BS_CUDA(cudaMallocHost(reinterpret_cast<void **>(&s->one_host), sizeof(int)));
     *s->one_host = 1;
 
@@ -1788,21 +1826,14 @@ static int set_external_forces(bs_sim *s, const float *f, bool wait)
         return fail(s, BS_E_STATE, "external forces are not available for batched ensembles");
     if (!f)
         return fail(s, BS_E_ARG, "bs_set_external_forces: null forces");
-    // Copied in stream order after the enqueued steps: straight from the caller's buffer when it
-    // is page-locked, else through the handle's pinned staging buffer. With wait (or a pageable
-    // buffer) the call returns when the copy is done, so the caller may reuse f.
-    const size_t bytes = sizeof(float) * 3 * static_cast<size_t>(s->n);
-    cudaPointerAttributes attr{};
-    const bool pinned = cudaPointerGetAttributes(&attr, f) == cudaSuccess && attr.type == cudaMemoryTypeHost;
-    if (!pinned)
-    {
-        cudaGetLastError(); // clear a pageable-pointer query error, if any
-        BS_CUDA(cudaStreamSynchronize(s->stream)); // the staging buffer may still feed an earlier copy
-        std::memcpy(s->ext_stage, f, bytes);
-    }
-    BS_CUDA(cudaMemcpyAsync(s->p.ext, pinned ? f : s->ext_stage, bytes, cudaMemcpyHostToDevice, s->stream));
+    // Copied in stream order after the enqueued steps: straight from the caller's buffer when it is
+    // page-locked, and then waited for if the caller may reuse it at once, else through the handle's own.
+    const bool pinned = memory_type(f) == cudaMemoryTypeHost;
+    const int rc = upload(s, s->p.ext, f, 3 * static_cast<size_t>(s->n), pinned);
+    if (rc)
+        return rc;
     BS_CUDA(cudaMemcpyAsync(&s->p.ctl->ext_pending, s->one_host, sizeof(int), cudaMemcpyHostToDevice, s->stream));
-    if (wait || !pinned)
+    if (wait && pinned)
         BS_CUDA(cudaStreamSynchronize(s->stream));
     return BS_OK;
 }
@@ -1822,19 +1853,30 @@ int bs_compute_forces(bs_sim *s)
     int rc = settle(s);
     if (rc)
         return rc;
-    if (!s->list_valid || (s->ctl_host->status & ST_STALE))
-    {
-        rc = rebuild_now(s);
-        if (rc)
-            return rc;
-    }
-    s->launches += launch_step(s->p, MODE_FORCES, s->stream);
+    const bool rebuild = !s->list_valid || (s->ctl_host->status & ST_STALE);
+    if (rebuild)
+        s->launches += launch_rebuild(s->p, s->stream);
+    s->launches += launch_step(s->p, MODE_FORCES, s->stream); // (does nothing if the rebuild raised a bit)
     BS_CUDA(cudaGetLastError());
     rc = read_ctl(s);
     if (rc)
         return rc;
-    if (s->ctl_host->status & ST_BARRIER)
-        return fail(s, BS_E_CUDA, "a grid barrier of the list rebuild timed out");
+    if (rebuild && (s->ctl_host->status & kRebuildBlocking))
+    {
+        rc = rebuild_now(s); // grows what was too small, or reports what is wrong
+        if (rc)
+            return rc;
+        s->launches += launch_step(s->p, MODE_FORCES, s->stream);
+        BS_CUDA(cudaGetLastError());
+        rc = read_ctl(s);
+        if (rc)
+            return rc;
+    }
+    if (rebuild)
+    {
+        s->list_valid = true;
+        s->since_rebuild = 0;
+    }
     if (s->ctl_host->status & ~ST_STALE)
         return fail(s, BS_E_STATE, "bs_compute_forces: device status not clean");
     return BS_OK;
@@ -1851,10 +1893,20 @@ static int get_vec(bs_sim *s, int what, float *out)
     const int rc = settle(s);
     if (rc)
         return rc;
-    s->launches += launch_unsort(s->p, what, s->staging, s->stream);
+    // the energies of the control block stay current: this kernel only reads the state
+    const bool current = s->ctl_read_at == s->launches;
+    const size_t bytes = sizeof(float) * 3 * s->n;
+    // small systems: the kernel writes the handle's page-locked buffer itself, one trip instead of two
+    const bool direct = bytes <= kDirectOut && memory_type(out) != cudaMemoryTypeDevice;
+    s->launches += launch_unsort(s->p, what, direct ? s->stage_h : s->staging, s->stream);
+    if (current)
+        s->ctl_read_at = s->launches;
     BS_CUDA(cudaGetLastError());
-    BS_CUDA(cudaMemcpyAsync(out, s->staging, sizeof(float) * 3 * s->n, cudaMemcpyDeviceToHost, s->stream));
+    if (!direct)
+        BS_CUDA(cudaMemcpyAsync(out, s->staging, bytes, cudaMemcpyDeviceToHost, s->stream));
     BS_CUDA(cudaStreamSynchronize(s->stream));
+    if (direct)
+        std::memcpy(out, s->stage_h, bytes);
     return BS_OK;
 }
 
@@ -1871,13 +1923,17 @@ static int set_state(bs_sim *s, const float *xyz, const float *vel)
     const float *src = xyz ? xyz : vel;
     if (!src)
         return fail(s, BS_E_ARG, "null input");
-    const int rc = settle(s);
+    int rc = settle(s);
     if (rc)
         return rc;
-    BS_CUDA(cudaMemcpyAsync(s->staging, src, sizeof(float) * 3 * s->n, cudaMemcpyHostToDevice, s->stream));
+    const bool pinned = memory_type(src) != cudaMemoryTypeUnregistered;
+    rc = upload(s, s->staging, src, 3 * static_cast<size_t>(s->n), pinned);
+    if (rc)
+        return rc;
     s->launches += launch_set_positions(s->p, xyz ? s->staging : nullptr, xyz ? nullptr : s->staging, s->stream);
     BS_CUDA(cudaGetLastError());
-    BS_CUDA(cudaStreamSynchronize(s->stream));
+    if (pinned)
+        BS_CUDA(cudaStreamSynchronize(s->stream));
     if (xyz)
         s->list_valid = false;
     return BS_OK;
@@ -2248,38 +2304,48 @@ int bs_get_spring_count(bs_sim *s, int64_t *count)
     return BS_OK;
 }
 
+// The spring and end of every directed entry of the caller-order table, on the device.
+static int spring_ids(bs_sim *s)
+{
+    if (s->sp_sid_d)
+        return BS_OK;
+    BS_CUDA(s->adj_dev.alloc(&s->sp_sid_d, s->csr_sid.size()));
+    BS_CUDA(cudaMemcpyAsync(s->sp_sid_d, s->csr_sid.data(), sizeof(unsigned int) * s->csr_sid.size(),
+                            cudaMemcpyHostToDevice, s->stream));
+    return BS_OK;
+}
+
 int bs_set_spring_parameters(bs_sim *s, const float *stiffness, const float *equilibrium)
 {
     if (!s)
         return fail(nullptr, BS_E_ARG, "null handle");
     if (!s->ready)
         return fail(s, BS_E_STATE, "call bs_setup first");
-    int rc = bs_synchronize(s);
+    // steps still enqueued run with the old parameters, and what they (or earlier ones) raised is reported
+    int rc = s->target > s->steps_done || s->ctl_host->status ? bs_synchronize(s) : BS_OK;
     if (rc)
         return rc;
     const size_t ns = s->sp_i.size();
     if (ns == 0)
         return BS_OK;
-    for (size_t t = 0; t < ns; ++t)
-    {
-        if (stiffness)
-            s->sp_k[t] = stiffness[t];
-        if (equilibrium)
-            s->sp_r0[t] = equilibrium[t];
-    }
-    const size_t nnz = 2 * ns;
-    std::vector<float> kk(nnz), rr(nnz);
-    for (size_t t = 0; t < ns; ++t)
-        for (int e = 0; e < 2; ++e)
+    rc = spring_ids(s);
+    if (rc)
+        return rc;
+    if (!s->sp_stage_d)
+        BS_CUDA(s->adj_dev.alloc(&s->sp_stage_d, 2 * ns));
+    const float *src[2] = {stiffness, equilibrium};
+    std::vector<float> *host[2] = {&s->sp_k, &s->sp_r0};
+    for (int q = 0; q < 2; ++q)
+        if (src[q])
         {
-            kk[s->csr_pos[2 * t + e]] = s->sp_k[t];
-            rr[s->csr_pos[2 * t + e]] = s->sp_r0[t];
+            std::memcpy(host[q]->data(), src[q], sizeof(float) * ns);
+            BS_CUDA(cudaMemcpyAsync(s->sp_stage_d + q * ns, host[q]->data(), sizeof(float) * ns, cudaMemcpyHostToDevice,
+                                    s->stream));
         }
-    BS_CUDA(cudaMemcpyAsync(const_cast<float *>(s->p.sp_k), kk.data(), sizeof(float) * nnz, cudaMemcpyHostToDevice,
-                            s->stream));
-    BS_CUDA(cudaMemcpyAsync(const_cast<float *>(s->p.sp_r0), rr.data(), sizeof(float) * nnz, cudaMemcpyHostToDevice,
-                            s->stream));
-    BS_CUDA(cudaStreamSynchronize(s->stream));
+    s->launches += launch_set_springs(s->p, 2 * static_cast<int>(ns), s->sp_sid_d, stiffness ? s->sp_stage_d : nullptr,
+                                      equilibrium ? s->sp_stage_d + ns : nullptr, s->stream);
+    BS_CUDA(cudaGetLastError());
+    BS_CUDA(cudaStreamSynchronize(s->stream)); // the handle's arrays may be written again by the next call
     s->list_valid = false; // the next rebuild copies them into the sorted spring table
     return BS_OK;
 }
@@ -2439,7 +2505,8 @@ int bs_adjoint(bs_sim *s, int32_t nsteps, int32_t checkpoint, const float *targe
     const size_t ns = s->sp_i.size();
     // Positions of every step kept when they take at most a quarter of the free device memory
     // (10,000 particles x 200 steps: 32 MB, twice that with precise positions).
-    bool keep_all = false;
+    bool keep_all = s->adj_seg_cap >= nsteps && s->adj_lx; // (an earlier run holds the room)
+    if (!keep_all)
     {
         size_t free_b = 0, total_b = 0;
         BS_CUDA(cudaMemGetInfo(&free_b, &total_b));
@@ -2451,14 +2518,13 @@ int bs_adjoint(bs_sim *s, int32_t nsteps, int32_t checkpoint, const float *targe
     // directed spring ids in the sorted spring table (filled by every rebuild from now on)
     if (!p.se_sid)
     {
-        unsigned int *d_sid = nullptr, *e_sid = nullptr;
-        BS_CUDA(s->adj_dev.alloc(&d_sid, s->csr_sid.size()));
+        rc = spring_ids(s);
+        if (rc)
+            return rc;
+        unsigned int *e_sid = nullptr;
         BS_CUDA(s->adj_dev.alloc(&e_sid, np * p.sp_maxdeg));
-        BS_CUDA(cudaMemcpyAsync(d_sid, s->csr_sid.data(), sizeof(unsigned int) * s->csr_sid.size(),
-                                cudaMemcpyHostToDevice, s->stream));
-        p.sp_sid = d_sid;
+        p.sp_sid = s->sp_sid_d;
         p.se_sid = e_sid;
-        s->sp_sid_d = d_sid;
         destroy_graph(s);
     }
     if (S > s->adj_ck_cap || seg_cap > s->adj_seg_cap || !s->adj_lx)
@@ -2479,7 +2545,7 @@ int bs_adjoint(bs_sim *s, int32_t nsteps, int32_t checkpoint, const float *targe
         BS_CUDA(s->dev.alloc(&s->adj_nu[1], np));
         BS_CUDA(s->dev.alloc(&s->adj_cx, np));
         BS_CUDA(s->dev.alloc(&s->adj_cv, np));
-        BS_CUDA(s->dev.alloc(&s->adj_target, np));
+        BS_CUDA(s->dev.alloc(&s->adj_target, n3));
         BS_CUDA(s->dev.alloc(&s->adj_gk, 2 * std::max<size_t>(ns, 1)));
         BS_CUDA(s->dev.alloc(&s->adj_gr0, 2 * std::max<size_t>(ns, 1)));
         BS_CUDA(s->dev.alloc(&s->adj_ok, std::max<size_t>(ns, 1)));
@@ -2489,15 +2555,8 @@ int bs_adjoint(bs_sim *s, int32_t nsteps, int32_t checkpoint, const float *targe
         BS_CUDA(s->dev.alloc(&s->adj_done, 1));
         BS_CUDA(cudaMemsetAsync(s->adj_done, 0, sizeof(unsigned int), s->stream));
     }
-    // the target, caller order
-    {
-        std::vector<float4> tg(np, make_float4(0.f, 0.f, 0.f, 0.f));
-        for (int64_t i = 0; i < s->n; ++i)
-            tg[i] = make_float4(target[3 * i], target[3 * i + 1], target[3 * i + 2], 0.f);
-        BS_CUDA(cudaMemcpyAsync(s->adj_target, tg.data(), sizeof(float4) * np, cudaMemcpyHostToDevice, s->stream));
-        BS_CUDA(cudaStreamSynchronize(s->stream));
-    }
-    rc = read_ctl(s);
+    const bool pinned = memory_type(target) != cudaMemoryTypeUnregistered;
+    rc = upload(s, s->adj_target, target, n3, pinned);
     if (rc)
         return rc;
     const Ctl saved = *s->ctl_host;
@@ -2575,20 +2634,18 @@ int bs_adjoint(bs_sim *s, int32_t nsteps, int32_t checkpoint, const float *targe
         s->ctl_host->steps = saved.steps;
         for (int k = 0; k < 8; ++k)
             s->ctl_host->energies[k] = saved.energies[k];
-        BS_CUDA(cudaMemcpy(s->p.ctl, s->ctl_host, sizeof(Ctl), cudaMemcpyHostToDevice));
-        BS_CUDA(cudaMemcpy(loss, s->adj_loss, sizeof(double), cudaMemcpyDeviceToHost));
+        BS_CUDA(cudaMemcpyAsync(s->p.ctl, s->ctl_host, sizeof(Ctl), cudaMemcpyHostToDevice, s->stream));
+        BS_CUDA(cudaMemcpyAsync(loss, s->adj_loss, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
         if (ns)
         {
-            BS_CUDA(cudaMemcpy(dL_dk, s->adj_ok, sizeof(float) * ns, cudaMemcpyDeviceToHost));
-            BS_CUDA(cudaMemcpy(dL_dr0, s->adj_or0, sizeof(float) * ns, cudaMemcpyDeviceToHost));
+            BS_CUDA(cudaMemcpyAsync(dL_dk, s->adj_ok, sizeof(float) * ns, cudaMemcpyDeviceToHost, s->stream));
+            BS_CUDA(cudaMemcpyAsync(dL_dr0, s->adj_or0, sizeof(float) * ns, cudaMemcpyDeviceToHost, s->stream));
         }
-        if (charges)
-        {
-            if (c.coulomb_enable)
-                BS_CUDA(cudaMemcpy(dL_dq, s->adj_gq, sizeof(float) * s->n, cudaMemcpyDeviceToHost));
-            else
-                std::memset(dL_dq, 0, sizeof(float) * s->n);
-        }
+        if (charges && c.coulomb_enable)
+            BS_CUDA(cudaMemcpyAsync(dL_dq, s->adj_gq, sizeof(float) * s->n, cudaMemcpyDeviceToHost, s->stream));
+        BS_CUDA(cudaStreamSynchronize(s->stream));
+        if (charges && !c.coulomb_enable)
+            std::memset(dL_dq, 0, sizeof(float) * s->n);
         return BS_OK;
     }
     return fail(s, BS_E_CAPACITY, "bs_adjoint: lists did not fit after repeated growth");

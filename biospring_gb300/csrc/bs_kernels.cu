@@ -481,6 +481,24 @@ int launch_set_charges(const Params &p, const float *q, cudaStream_t st)
     return 1;
 }
 
+__global__ void k_set_springs(Params p, int nnz, const unsigned int *sid, const float *k, const float *r0)
+{
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= nnz)
+        return;
+    const unsigned int t = sid[e] >> 1; // 2 * spring + end
+    if (k)
+        const_cast<float *>(p.sp_k)[e] = k[t];
+    if (r0)
+        const_cast<float *>(p.sp_r0)[e] = r0[t];
+}
+
+int launch_set_springs(const Params &p, int nnz, const unsigned int *sid, const float *k, const float *r0, cudaStream_t st)
+{
+    k_set_springs<<<(nnz + 255) / 256, 256, 0, st>>>(p, nnz, sid, k, r0);
+    return 1;
+}
+
 // Adds one particle's external force for the next step and marks it pending (bs_set_force).
 __global__ void k_ext_add(Params p, long long i, float fx, float fy, float fz)
 {

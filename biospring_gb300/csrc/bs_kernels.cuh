@@ -117,6 +117,8 @@ inline bool lean_step(const Params &p)
 int launch_ext_add(const Params &p, long long i, float fx, float fy, float fz, cudaStream_t stream);
 int launch_set_burying(const Params &p, const float *burying, cudaStream_t stream);
 int launch_set_charges(const Params &p, const float *q, cudaStream_t st);
+// new stiffness and rest length (nullable, by spring) into the nnz entries of the caller-order spring table
+int launch_set_springs(const Params &p, int nnz, const unsigned int *sid, const float *k, const float *r0, cudaStream_t st);
 int launch_unsort(const Params &p, int what, float *out3, cudaStream_t stream);
 int launch_diag_cells(const Params &p, float cutoff, float skin, uint32_t need_flag, long long *out,
                       cudaStream_t stream);
@@ -143,7 +145,7 @@ int launch_adj_step(const Params &p, const AdjState &a, cudaStream_t stream);
 // resident at once (0: none is)
 cudaError_t adj_run_lanes(const Params &p, int *lanes);
 cudaError_t launch_adj_run(const Params &p, const AdjState &a, int count, int lanes, cudaStream_t stream);
-int launch_adj_init(const Params &p, const AdjState &a, const float4 *target, double *blk, unsigned int *done,
+int launch_adj_init(const Params &p, const AdjState &a, const float *target, double *blk, unsigned int *done,
                     double *loss, cudaStream_t stream);
 int launch_adj_permute(const Params &p, const AdjState &a, float4 *cx, float4 *cv, int dir, cudaStream_t stream);
 int launch_adj_save(const Params &p, float4 *dst, float4 *dst_lo, cudaStream_t stream);
