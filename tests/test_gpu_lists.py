@@ -34,10 +34,12 @@ def _beads(n, density, seed, flat=False):
 
 def _check(s, terms):
     net, orc = gpu_network(s), po.Oracle(s)
+    found = 0
     for term in terms:
         got, ref = net.getPairs(term), orc.pairs(term).astype(np.int64)
-        assert ref.shape[0] > 0
+        found += ref.shape[0]
         np.testing.assert_array_equal(got, ref)
+    assert found > 0
     net.close()
     orc.close()
 
@@ -75,6 +77,21 @@ def test_crowded_corner():
     s.xyz[near] *= np.float32(0.5)  # eight times the density: rows past their first capacity
     s.config.update(steric_enable=1, steric_mode=1, steric_cutoff=10.0, coulomb_enable=1, coulomb_cutoff=10.0)
     _check(s, (0, 1))
+
+
+@pytest.mark.parametrize("n", [63999, 64000, 64161])
+def test_sparse(n):
+    """Few particles a cell: a warp a home below 64,000 particles, a thread a home from there on."""
+    s = _beads(n, 0.004, n)
+    s.config.update(spring_enable=1, steric_enable=1, steric_mode=1, steric_cutoff=9.0, coulomb_enable=1,
+                    coulomb_cutoff=8.0, hydrophobicity_enable=1, hydrophobicity_cutoff=9.0, list_skin=0.5)
+    _check(s, (0, 1, 2))
+
+
+def test_sparse_wide_offsets():
+    s = _beads(120000, 0.004, 8, flat=True)
+    s.config.update(spring_enable=1, steric_enable=1, steric_mode=1, steric_cutoff=9.0)
+    _check(s, (0,))
 
 
 def test_wide_offsets():
