@@ -1582,14 +1582,12 @@ int bs_setup(bs_sim *s, const bs_config *cfg)
     p.k_hydro_e = static_cast<float>(kAvogadro * 1.0E-3);
 
     BS_CUDA(order_blocks(p, &p.order_blocks));
-    bool fits = false;
-    BS_CUDA(run_fits(p, &fits));
-    if (fits)
+    BS_CUDA(run_fits(p));
+    if (p.run_on)
     {
         BS_CUDA(s->dev.alloc(&p.run_arrive, 1));
         BS_CUDA(cudaMemsetAsync(p.run_arrive, 0, sizeof(unsigned int), s->stream));
         BS_CUDA(s->dev.alloc(&p.run_probe, 16 * static_cast<size_t>(run_blocks(p))));
-        p.run_on = 1;
     }
 
     s->ready = true;

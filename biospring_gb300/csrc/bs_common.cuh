@@ -205,6 +205,7 @@ struct Params
     Ctl *ctl;
     // kernels of several steps (bs_run.cu)
     int run_on;               // the system's step grid is resident at once: k_run takes its steps
+    int run_hold;             // the form of k_run: rows held in registers at 2 or 3 blocks per SM, or not (0)
     unsigned int *run_arrive; // grid-barrier word, 0 between launches
     float *run_probe;         // [2][blocks][8] the probe's per-block sums, by the parity of the step
     // configuration

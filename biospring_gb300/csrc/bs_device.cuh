@@ -736,13 +736,13 @@ __device__ __forceinline__ void steric_forces_batched(const Params &p, int s, in
 // Springs of slot s, lane t of T, in passes of kGatherU entries per lane (entries t + T u of the
 // ELL row, the same entries in the same order as spring_forces): the U entries' columns are read
 // first, then the U partner positions together.
-template <int T, class POS>
+template <int T, class POS, class HELD>
 __device__ __forceinline__ void spring_forces_batched(const Params &p, int s, int t, float4 pi,
                                                       const POS pos, float &fx, float &fy, float &fz,
-                                                      float &e)
+                                                      float &e, const HELD &held)
 {
     constexpr int U = kGatherU;
-    const int deg = p.se_deg[s];
+    const int deg = HELD::on ? held.deg : p.se_deg[s];
     const size_t stride = static_cast<size_t>(p.npad);
     for (int k0 = t; k0 < deg; k0 += T * U)
     {
@@ -756,7 +756,13 @@ __device__ __forceinline__ void spring_forces_batched(const Params &p, int s, in
             c[u] = kEntryInactive;
             kk[u] = 0.0f;
             r0[u] = 0.0f;
-            if (k < deg)
+            if (HELD::on && k0 == t)
+            {
+                c[u] = held.c[u];
+                kk[u] = held.k[u];
+                r0[u] = held.r[u];
+            }
+            else if (k < deg)
             {
                 const size_t at = static_cast<size_t>(k) * stride + s;
                 c[u] = __ldg(&p.se_col[at]);
@@ -1057,6 +1063,63 @@ template <int T> __device__ __forceinline__ float group_sum(float v)
     return v;
 }
 
+// What a kernel of several steps keeps in registers from step to step, as long as the lists stay the same:
+// the particle's flags and steric factor, the lane's first entries of the steric row (16-bit) and of the
+// spring row. Each was a dependent read in every step, after a barrier that empties the L1.
+struct NoHeld
+{
+    static constexpr bool on = false;
+    int deg;
+    unsigned int c[kGatherU];
+    float k[kGatherU], r[kGatherU];
+};
+template <int T> struct RowHeld
+{
+    static constexpr bool on = true;
+    unsigned int flags;
+    float fhi;
+    int cnt;
+    uint2 w;
+    int deg;
+    unsigned int c[kGatherU];
+    float k[kGatherU], r[kGatherU];
+    __device__ __forceinline__ RowHeld(const Params &p, int s, int t, int lb)
+        : flags(PF_STATIC), fhi(0.0f), cnt(-1), w(make_uint2(0u, 0u)), deg(0)
+    {
+#pragma unroll
+        for (int u = 0; u < kGatherU; ++u)
+        {
+            c[u] = kEntryInactive;
+            k[u] = r[u] = 0.0f;
+        }
+        if (s >= p.n)
+            return;
+        flags = p.flags[lb][s];
+        fhi = p.fhi[lb][s];
+        if (p.steric_on && p.pl16)
+        {
+            const PairList &L = p.pl[0];
+            cnt = L.cnt[s];
+            if (kGatherU * t < L.cap)
+                w = __ldg(reinterpret_cast<const uint2 *>(reinterpret_cast<const short *>(L.idx) +
+                                                        static_cast<size_t>(s) * L.cap + kGatherU * t));
+        }
+        if (p.spring_on)
+        {
+            deg = p.se_deg[s];
+#pragma unroll
+            for (int u = 0; u < kGatherU; ++u)
+                if (t + u * T < deg)
+                {
+                    const size_t at = static_cast<size_t>(t + u * T) * p.npad + s;
+                    c[u] = __ldg(&p.se_col[at]);
+                    k[u] = __ldg(&p.se_k[at]);
+                    r[u] = __ldg(&p.se_r0[at]);
+                }
+        }
+    }
+};
+
 // One particle of one step (or of one force evaluation), lane t of the T consecutive lanes that
 // share slot s: each lane takes every T-th entry of the particle's spring row and pair lists, the
 // group sums its partial forces with shuffles, and the group's first lane adds the per-particle
@@ -1067,10 +1130,10 @@ template <int T> __device__ __forceinline__ float group_sum(float v)
 // Coulomb rows walked by the whole warp. The batched kernel leaves both out (fewer live registers
 // under its 64-register budget: with them its spills grew and its step slowed by 7%); it walks
 // Coulomb rows with the particle's own lanes (the same pairs, summed in another order).
-template <int MODE, int SM, int T, bool SINGLE = true, bool LEAN = false, class POS = PosConst>
+template <int MODE, int SM, int T, bool SINGLE = true, bool LEAN = false, class POS = PosConst, class HELD = NoHeld>
 __device__ __forceinline__ int particle_step(const Params &p, const int s, const int t, const int send,
                                              const int sb, const int lb, const bool ext_on, const float4 *probe,
-                                             float (&eacc)[6])
+                                             float (&eacc)[6], const HELD &held = HELD())
 {
     const POS pos{p.pos[sb]};
     const bool lead = t == 0;
@@ -1091,9 +1154,19 @@ __device__ __forceinline__ int particle_step(const Params &p, const int s, const
     if (s < send)
     {
         pi = pos[s];
-        fi = p.flags[lb][s];
-        fhi_i = p.fhi[lb][s];
-        if (kHoist && p.steric_on && p.lj_uniform && p.pl16)
+        if constexpr (HELD::on)
+        {
+            fi = held.flags;
+            fhi_i = held.fhi;
+            cnt0 = held.cnt;
+            w0 = held.w;
+        }
+        else
+        {
+            fi = p.flags[lb][s];
+            fhi_i = p.fhi[lb][s];
+        }
+        if (!HELD::on && kHoist && p.steric_on && p.lj_uniform && p.pl16)
         {
             const PairList &L = p.pl[0];
             cnt0 = L.cnt[s];
@@ -1113,7 +1186,8 @@ __device__ __forceinline__ int particle_step(const Params &p, const int s, const
             else if ((SINGLE && BS_GATHER) || (!SINGLE && BS_GATHER_BATCH))
             {
                 if (p.pl16)
-                    steric_forces_batched<SM, T, true, false>(p, s, t, pi, fhi_i, pos, p.fhi[lb], sx, sy, sz, es);
+                    steric_forces_batched<SM, T, true, false>(p, s, t, pi, fhi_i, pos, p.fhi[lb], sx, sy, sz, es,
+                                                              HELD::on ? cnt0 : -1, w0);
                 else
                     steric_forces_batched<SM, T, false, false>(p, s, t, pi, fhi_i, pos, p.fhi[lb], sx, sy, sz, es);
             }
@@ -1135,7 +1209,7 @@ __device__ __forceinline__ int particle_step(const Params &p, const int s, const
         {
             float sx = 0.f, sy = 0.f, sz = 0.f, es = 0.f;
             if ((SINGLE && BS_GATHER) || (!SINGLE && BS_GATHER_BATCH))
-                spring_forces_batched<T>(p, s, t, pi, pos, sx, sy, sz, es);
+                spring_forces_batched<T>(p, s, t, pi, pos, sx, sy, sz, es, held);
             else
                 spring_forces<T>(p, s, t, pi, pos, sx, sy, sz, es);
             const float kf = p.k_spring_f * p.spring_scale;

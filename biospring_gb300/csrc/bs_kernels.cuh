@@ -101,7 +101,7 @@ int launch_steps(const Params &p, int count, cudaStream_t stream);
 // (save, save_lo, nullable: the positions every step starts from and their remainders, npad a step)
 cudaError_t launch_run(const Params &p, int count, cudaStream_t stream, float4 *save = nullptr,
                        float4 *save_lo = nullptr);
-cudaError_t run_fits(const Params &p, bool *fits);
+cudaError_t run_fits(Params &p); // sets run_on and run_hold
 int run_blocks(const Params &p);
 // Steps of one launch (10 in the default schedule) and the polls after which a barrier gives up (some
 // seconds; a meeting takes about a microsecond).

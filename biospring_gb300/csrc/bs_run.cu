@@ -10,10 +10,17 @@
 // results are the same bit for bit. The probe's reaction is summed block by block, and every block then
 // computes the probe's step itself, so it costs no barrier of its own.
 //
+// Where registers allow, the lanes keep the first entries of their steric and spring rows from step to step:
+// after a barrier, which empties the L1, each was a dependent read of its own. Calls with and without: Calpha
+// network of 2,000 792 -> 706 us (2 blocks an SM; 729 with 3), training step of 10,000 4,507 -> 4,260 us (3
+// blocks), Lennard-Jones 5,003 316 -> 304 us, 6,007 with the probe 510 -> 502 us.
+//
 // Bound: the chain of dependent loads of a step, then the barrier. Measured, a call of 50 to 100 steps
 // with its rebuilds, a kernel a step against this one: Calpha network of 2,000 1,423 -> 905 us (100
 // steps), Lennard-Jones beads 5,003 431 -> 339 us (20), receptor and ligand of 6,007 with the probe 677 ->
 // 530 us (20), membrane of 20,000 with four bodies 1,460 -> 1,284 us (50).
+
+#include <type_traits>
 
 #include "bs_rigid.cuh"
 
@@ -67,8 +74,10 @@ __device__ __forceinline__ void probe_step(const Params &p, const float *part, f
     __syncthreads();
 }
 
-template <int SM, int T, bool LEAN>
-__global__ void __launch_bounds__(kStepKernelBlock, kStepMinBlocks) k_run(Params p, int count, float4 *save, float4 *save_lo)
+// HOLD: the lanes keep the first entries of their rows in registers (RowHeld); 2 or 3 is also the blocks an SM
+// that leave registers enough for it (128 or 80 a thread).
+template <int SM, int T, bool LEAN, int HOLD>
+__global__ void __launch_bounds__(kStepKernelBlock, HOLD ? HOLD : kStepMinBlocks) k_run(Params p, int count, float4 *save, float4 *save_lo)
 {
     Ctl *ctl = p.ctl;
     if (status_of(ctl) != 0)
@@ -89,6 +98,13 @@ __global__ void __launch_bounds__(kStepKernelBlock, kStepMinBlocks) k_run(Params
         }
         __syncthreads();
     }
+    using Held = std::conditional_t<HOLD != 0, RowHeld<T>, NoHeld>;
+    const Held held = [&] {
+        if constexpr (HOLD != 0)
+            return RowHeld<T>(p, g / T, g % T, lb);
+        else
+            return NoHeld();
+    }();
     float e[6];
     unsigned int gen = 0;
     int k = 0, go = 1;
@@ -105,8 +121,8 @@ __global__ void __launch_bounds__(kStepKernelBlock, kStepMinBlocks) k_run(Params
             if (!LEAN && save_lo)
                 save_lo[at] = p.pos_lo[sb][g / T];
         }
-        int pend = particle_step<MODE_STEP, SM, T, true, LEAN, PosShared>(p, g / T, g % T, p.n, sb, lb, ext && k == 0,
-                                                                          prb, e);
+        int pend = particle_step<MODE_STEP, SM, T, true, LEAN, PosShared, Held>(p, g / T, g % T, p.n, sb, lb,
+                                                                                 ext && k == 0, prb, e, held);
         float *part = p.run_probe + static_cast<size_t>(k & 1) * 8 * gridDim.x; // read until the next step's barrier
         if (probe)
         {
@@ -166,35 +182,37 @@ __global__ void __launch_bounds__(kStepKernelBlock, kStepMinBlocks) k_run(Params
     }
 }
 
-template <int SM> const void *run_fn(int lanes, bool lean)
+template <int SM, int T, int HOLD> const void *run_lean(bool lean)
 {
-    switch (lanes)
-    {
-    case 4:
-        return lean ? reinterpret_cast<const void *>(&k_run<SM, 4, true>) : reinterpret_cast<const void *>(&k_run<SM, 4, false>);
-    case 8:
-        return lean ? reinterpret_cast<const void *>(&k_run<SM, 8, true>) : reinterpret_cast<const void *>(&k_run<SM, 8, false>);
-    case 16:
-        return lean ? reinterpret_cast<const void *>(&k_run<SM, 16, true>)
-                    : reinterpret_cast<const void *>(&k_run<SM, 16, false>);
-    default:
-        return nullptr;
-    }
+    return lean ? reinterpret_cast<const void *>(&k_run<SM, T, true, HOLD>)
+                : reinterpret_cast<const void *>(&k_run<SM, T, false, HOLD>);
+}
+
+// The forms there are: with 16 lanes a particle the rows held at 2 or 3 blocks an SM, with 8 lanes at 3. With 4
+// lanes the held entries are too small a part of the rows (a membrane of 20,000 got 2% slower).
+template <int SM> const void *run_fn(int lanes, bool lean, int hold)
+{
+    if (lanes == 16)
+        return hold == 2 ? run_lean<SM, 16, 2>(lean) : (hold == 3 ? run_lean<SM, 16, 3>(lean) : run_lean<SM, 16, 0>(lean));
+    if (lanes == 8)
+        return hold == 2 ? nullptr : (hold == 3 ? run_lean<SM, 8, 3>(lean) : run_lean<SM, 8, 0>(lean));
+    return lanes == 4 && hold == 0 ? run_lean<SM, 4, 0>(lean) : nullptr;
 }
 
 const void *run_kernel(const Params &p)
 {
     const bool lean = lean_step(p);
+    const int hold = p.run_hold;
     switch (p.steric_mode)
     {
     case BS_STERIC_LINEAR:
-        return run_fn<BS_STERIC_LINEAR>(p.step_lanes, lean);
+        return run_fn<BS_STERIC_LINEAR>(p.step_lanes, lean, hold);
     case BS_STERIC_LJ_12_6_AMBER:
-        return run_fn<BS_STERIC_LJ_12_6_AMBER>(p.step_lanes, lean);
+        return run_fn<BS_STERIC_LJ_12_6_AMBER>(p.step_lanes, lean, hold);
     case BS_STERIC_LJ_8_6_LEWITT:
-        return run_fn<BS_STERIC_LJ_8_6_LEWITT>(p.step_lanes, lean);
+        return run_fn<BS_STERIC_LJ_8_6_LEWITT>(p.step_lanes, lean, hold);
     case BS_STERIC_LJ_8_6_ZACHARIAS:
-        return run_fn<BS_STERIC_LJ_8_6_ZACHARIAS>(p.step_lanes, lean);
+        return run_fn<BS_STERIC_LJ_8_6_ZACHARIAS>(p.step_lanes, lean, hold);
     default:
         return nullptr;
     }
@@ -207,20 +225,27 @@ int run_blocks(const Params &p)
     return static_cast<int>((static_cast<long long>(p.n) * p.step_lanes + kStepKernelBlock - 1) / kStepKernelBlock);
 }
 
-cudaError_t run_fits(const Params &p, bool *fits)
+cudaError_t run_fits(Params &p)
 {
-    *fits = false;
-    const void *fn = run_kernel(p);
-    int dev = 0, sms = 0, coop = 0, per_sm = 0;
+    p.run_on = p.run_hold = 0;
+    int dev = 0, sms = 0, coop = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess)
         e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess)
         e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-    if (e != cudaSuccess || !fn || !coop || p.nsys > 0)
-        return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kStepKernelBlock, 0);
-    *fits = e == cudaSuccess && run_blocks(p) <= per_sm * sms;
+    // the form with the most registers that is resident at once
+    const int forms[3] = {2, 3, 0};
+    for (int f = 0; f < 3 && !p.run_on && e == cudaSuccess && coop && p.nsys == 0; ++f)
+    {
+        p.run_hold = forms[f];
+        const void *fn = run_kernel(p);
+        if (!fn)
+            continue;
+        int per_sm = 0;
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kStepKernelBlock, 0);
+        p.run_on = e == cudaSuccess && run_blocks(p) <= per_sm * sms;
+    }
     return e;
 }
 

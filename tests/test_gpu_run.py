@@ -1,7 +1,7 @@
 """The kernel of several steps (one cooperative launch between two list rebuilds) against the same steps
 launched one kernel at a time: positions, velocities, energies and the step count bit for bit, at the
 edges of its blocks and of its range (16 lanes a particle below 8,000, 8 below 20,000, 4 up to the 38,912
-that 608 resident blocks hold), across stale lists and with bodies. With the probe, whose reaction is summed
+that 608 resident blocks hold; rows held in registers up to 4,864 and 7,296 with 16 lanes, 14,592 with 8), across stale lists and with bodies. With the probe, whose reaction is summed
 in another order (float-float, then rounded once), positions agree to 1e-6 A."""
 
 from __future__ import annotations
@@ -52,7 +52,8 @@ def _system(n):
     return s
 
 
-@pytest.mark.parametrize("n", [1, 16, 17, 300, 7999, 8001, 19456, 19457, 20000, 38912, 38913])
+@pytest.mark.parametrize("n", [1, 16, 17, 300, 4864, 4865, 7296, 7297, 7999, 8001, 14592, 14593, 19456, 19457, 20000, 38912,
+                               38913])
 def test_same_bits_as_single_steps(n):
     s = _system(n)
     a, b = gpu_network(s), gpu_network(s)
