@@ -103,6 +103,7 @@ struct bs_sim
     // growable buffers (pair lists, grid arrays), freed on regrowth
     unsigned int *pl_idx[kLists] = {nullptr, nullptr, nullptr, nullptr};
     int *cell_buf[2] = {nullptr, nullptr};
+    unsigned long long *cell_bin = nullptr;
     // batched ensembles: caller's partition into systems (empty: one system)
     std::vector<int64_t> sys_off;
     BatchShape shape{256, 4, 1};
@@ -297,6 +298,9 @@ void free_growable(bs_sim *s)
             cudaFree(s->cell_buf[k]);
         s->cell_buf[k] = nullptr;
     }
+    if (s->cell_bin)
+        cudaFree(s->cell_bin);
+    s->cell_bin = nullptr;
 }
 
 // (Re)allocates the three pair lists and the cell arrays for the given capacities. The stream
@@ -316,12 +320,17 @@ int alloc_lists(bs_sim *s, const int caps[kLists], int cell_cap)
         p.pl[t].idx = s->pl_idx[t];
         p.pl[t].cap = cap;
     }
+    // (four cells more: the counts are read four at a time)
     for (int k = 0; k < 2; ++k)
-        BS_CUDA(cudaMalloc(reinterpret_cast<void **>(&s->cell_buf[k]), (static_cast<size_t>(cell_cap) + 1) * sizeof(int)));
-    BS_CUDA(cudaMemsetAsync(s->cell_buf[0], 0, (static_cast<size_t>(cell_cap) + 1) * sizeof(int), s->stream));
+        BS_CUDA(cudaMalloc(reinterpret_cast<void **>(&s->cell_buf[k]), (static_cast<size_t>(cell_cap) + 4) * sizeof(int)));
+    BS_CUDA(cudaMemsetAsync(s->cell_buf[0], 0, (static_cast<size_t>(cell_cap) + 4) * sizeof(int), s->stream));
     p.cell_cnt = s->cell_buf[0];
     p.cell_start = s->cell_buf[1];
     p.cell_cap = cell_cap;
+    const size_t bins = s->sys_off.empty() ? order_bins(p) : 0;
+    if (bins > 0)
+        BS_CUDA(cudaMalloc(reinterpret_cast<void **>(&s->cell_bin), bins * sizeof(unsigned long long)));
+    p.cell_bin = s->cell_bin;
     destroy_graph(s);
     return BS_OK;
 }
@@ -1222,8 +1231,8 @@ int bs_setup(bs_sim *s, const bs_config *cfg)
     BS_CUDA(s->dev.alloc(&p.tmp_key, npad));
     BS_CUDA(s->dev.alloc(&p.cell_at, npad));
     BS_CUDA(s->dev.alloc(&p.tile_sum, kOrderMaxBlocks));
-    BS_CUDA(s->dev.alloc(&p.order_sync, 2));
-    BS_CUDA(cudaMemsetAsync(p.order_sync, 0, 2 * sizeof(unsigned int), s->stream));
+    BS_CUDA(s->dev.alloc(&p.order_sync, 3));
+    BS_CUDA(cudaMemsetAsync(p.order_sync, 0, 3 * sizeof(unsigned int), s->stream));
     s->step_blocks = static_cast<int>((static_cast<long long>(p.n) * 16 + kStepBlock - 1) / kStepBlock);
     p.blk_cap = s->step_blocks;
     BS_CUDA(s->dev.alloc(&p.blk_energy, energy_scratch_doubles(s->step_blocks)));

@@ -194,7 +194,8 @@ struct Params
     int cell_cap;
     int2 *cell_at;            // [npad] cell of each particle in the old order, its place of arrival there
     int *tile_sum;            // [kOrderMaxBlocks] cell totals of each block's share in the cell scan
-    unsigned int *order_sync; // [2] k_order's grid-barrier word and count of finished blocks, 0 between launches
+    unsigned long long *cell_bin; // [cells][64] order keys by cell, where k_order takes the short way
+    unsigned int *order_sync; // [3] k_order's grid-barrier word, finished blocks, full bin; 0 between launches
     int order_blocks;         // its grid, resident at once
     int pl_sparse;            // build the pair lists one warp per particle (few particles per cell)
     int lists_off;            // no nonbonded term is on: no pair lists, the grid only orders the particles

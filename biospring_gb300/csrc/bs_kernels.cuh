@@ -91,6 +91,7 @@ enum StepMode
 int launch_rebuild(const Params &p, cudaStream_t stream);
 cudaError_t launch_order(const Params &p, cudaStream_t stream); // bs_order.cu
 cudaError_t order_blocks(const Params &p, int *blocks);
+size_t order_bins(const Params &p); // entries of Params::cell_bin (single systems)
 int launch_pairlist(const Params &p, cudaStream_t stream); // bs_list.cu
 int launch_step(const Params &p, int mode, cudaStream_t stream);      // step kernel, then the bodies
 int launch_step_only(const Params &p, int mode, cudaStream_t stream); // the step kernel alone

@@ -10,7 +10,7 @@ import numpy as np
 import pytest
 
 from biospring_gb300 import workloads as W
-from helpers import gpu_network
+from helpers import gpu_network, rel_l2
 from oracle import pyoracle as po
 
 pytestmark = pytest.mark.gpu
@@ -86,6 +86,33 @@ def test_sparse(n):
     s.config.update(spring_enable=1, steric_enable=1, steric_mode=1, steric_cutoff=9.0, coulomb_enable=1,
                     coulomb_cutoff=8.0, hydrophobicity_enable=1, hydrophobicity_cutoff=9.0, list_skin=0.5)
     _check(s, (0, 1, 2))
+
+
+@pytest.mark.parametrize("n,density", [(8000, 0.0005), (8000, 0.0008), (65535, 0.02), (65536, 0.02)])
+def test_cell_order(n, density):
+    """The cell order by placed keys and by bins: more and fewer than the 4,096 cells of the short way, and
+    65,535 and 65,536 particles. The forces hang on the spring table of the new order (1e-5 relative, as the
+    other force checks)."""
+    s = _beads(n, density, n + 1)
+    s.config.update(spring_enable=1, steric_enable=1, steric_mode=1, steric_cutoff=9.0 if density > 0.01 else 17.0)
+    net, orc = gpu_network(s), po.Oracle(s)
+    np.testing.assert_array_equal(net.getPairs(0), orc.pairs(0).astype(np.int64))
+    net.computeForces()
+    orc.compute_forces()
+    assert rel_l2(net.getForces(), orc.forces(), s.is_static == 0) < 1e-5  # a static particle gets none
+    net.close()
+    orc.close()
+
+
+def test_full_bins():
+    """More than the 64 particles of a bin in one cell."""
+    rng = np.random.default_rng(12)
+    x = rng.uniform(0.0, 6.0, (600, 3)).astype(np.float32)
+    x[300:] += np.float32(100.0)
+    s = W.System("clumps", x, np.zeros((0, 2), np.int32), np.zeros(0, np.float32), np.zeros(0, np.float32), {})
+    s.radius, s.epsilon = np.full(600, 0.5, np.float32), np.full(600, 0.1, np.float32)
+    s.config.update(spring_enable=0, steric_enable=1, steric_mode=1, steric_cutoff=9.0)
+    _check(s, (0,))
 
 
 def test_sparse_wide_offsets():
