@@ -14,7 +14,7 @@ buffers: per step, external forces H2D from pinned memory, one bs_step call, ene
 Two more figures ride on the same line (rank 0, one GPU):
   batched  512 independent Calpha networks (sizes log-uniform in 200..20,000, ~2.1M particles),
            springs < 10 A, linear steric 8 A, viscosity, rebuild every 10 steps, stepped by the
-           persistent clustered kernel with the autotuned shape, against the same systems stepped
+           persistent kernel with the autotuned shape, against the same systems stepped
            one after another through the single-system path (inputs larger than L2);
   adjoint  loss and dL/dk, dL/dr0 of all springs of a 10,000-particle network after 200 steps with
            checkpoints every 20 (precise positions), timed against the plain 200-step forward of
@@ -59,7 +59,7 @@ CTL_BYTES = 272                       # device control block (status, step count
 # DRAM bytes (read + write) of one k_step launch on this workload after an L2 flush, from one ncu
 # capture of dram__bytes_read.sum + dram__bytes_write.sum, and the digest of the step kernel's
 # sources that capture ran on: when the sources have changed since, the line marks the figure stale.
-STEP_KERNEL_TRAFFIC = {"bytes": 69.48992e6 + 1.682176e6, "sources_sha": "d0671f577e273adc", "captured": "2026-12-04"}
+STEP_KERNEL_TRAFFIC = {"bytes": 69.496064e6 + 1.169408e6, "sources_sha": "49d474a01f21f92c", "captured": "2026-12-05"}
 STEP_KERNEL_SOURCES = ("biospring_gb300/csrc/bs_device.cuh", "biospring_gb300/csrc/bs_kernels.cu",
                        "biospring_gb300/csrc/bs_kernels.cuh", "biospring_gb300/csrc/bs_common.cuh")
 DIELECTRIC_NOTE = ("Coulomb eps = 4r (distance-dependent), as the 100k configuration states; the reference's "

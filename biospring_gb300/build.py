@@ -24,7 +24,8 @@ LIB = os.path.join(PKG, "libbiospring_gb300.so")
 SYNTH = os.path.join(PKG, "libbs_synth.so")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-CUDA_SOURCES = ["bs_kernels.cu", "bs_run.cu", "bs_order.cu", "bs_list.cu", "bs_batch.cu", "bs_adjoint.cu", "bs_rigid.cu", "bs_capi.cu", "bs_noalloc.cu"]
+CUDA_SOURCES = ["bs_kernels.cu", "bs_run.cu", "bs_run_linear.cu", "bs_run_amber.cu", "bs_run_lewitt.cu",
+                "bs_run_zacharias.cu", "bs_order.cu", "bs_list.cu", "bs_batch.cu", "bs_adjoint.cu", "bs_rigid.cu", "bs_capi.cu", "bs_noalloc.cu"]
 HOST_SOURCES = ["bs_msp.cpp", "bs_field.cpp", "bs_nc.cpp", "bs_xtc.cpp"]
 
 

@@ -1552,8 +1552,9 @@ int bs_setup(bs_sim *s, const bs_config *cfg)
     p.visc_on = c.viscosity_enable != 0;
     p.steric_mode = c.steric_mode;
     // lanes per particle: the fewest of 4, 8, 16 that still give the GPU some 64-80k threads
-    // (measured: 4 lanes from 20k particles, 8 from 8k, 16 below); BS_STEP_LANES overrides
-    p.step_lanes = n >= 20000 ? 4 : (n >= 8000 ? 8 : 16);
+    // (measured: 4 lanes from 20k particles, 8 from 8k, 16 below; 8 lanes end at 19,456, where 608 resident
+    // blocks hold the whole step and k_run takes it); BS_STEP_LANES overrides
+    p.step_lanes = n > 19456 ? 4 : (n >= 8000 ? 8 : 16);
     if (const char *env = std::getenv("BS_STEP_LANES"))
     {
         const int v = std::atoi(env);
@@ -1590,6 +1591,7 @@ int bs_setup(bs_sim *s, const bs_config *cfg)
     p.k_imp_f = static_cast<float>(kImpForceConvert);
     p.k_hydro_e = static_cast<float>(kAvogadro * 1.0E-3);
 
+    BS_CUDA(load_step_kernels());
     BS_CUDA(order_blocks(p, &p.order_blocks));
     BS_CUDA(run_fits(p));
     if (p.run_on)

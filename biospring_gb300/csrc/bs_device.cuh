@@ -18,9 +18,8 @@ namespace
 __device__ __forceinline__ int status_of(const Ctl *c) { return *(volatile const int *)&c->status; }
 
 // Programmatic dependent launch: lets the next kernel of the stream begin launching now, then waits
-// until the previous kernel has completed and its writes are visible. The launch of the next
-// kernel thus overlaps this one; both instructions are no-ops for a kernel launched without the
-// programmatic-serialization attribute. Every kernel of the rebuild and step chains calls it first.
+// until the previous kernel has completed and its writes are visible. Both instructions are no-ops where
+// neither kernel was launched with the programmatic-serialization attribute.
 __device__ __forceinline__ void pdl_enter()
 {
 #if BS_PDL

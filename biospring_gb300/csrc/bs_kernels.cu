@@ -360,41 +360,12 @@ __global__ void __launch_bounds__(kStepBlock) k_diag_pairs(Params p, int term, l
 
 } // namespace
 
-// Launches a kernel of the rebuild or step chain; with BS_PDL set, with programmatic stream
-// serialisation, so that it may start launching while its predecessor runs (it waits in pdl_enter).
 template <typename... KArgs, typename... Args>
 static void launch_plain(void (*kern)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
                          Args &&...args)
 {
     kern<<<grid, block, smem, st>>>(std::forward<Args>(args)...);
 }
-
-template <typename... KArgs, typename... Args>
-static void launch_chain(void (*kern)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
-                         Args &&...args)
-{
-#if BS_PDL
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
-#else
-    kern<<<grid, block, smem, st>>>(std::forward<Args>(args)...);
-#endif
-}
-
-#if BS_PDL_STEP
-#define BS_STEP_LAUNCH launch_chain
-#else
-#define BS_STEP_LAUNCH launch_plain
-#endif
 
 int launch_rebuild(const Params &p, cudaStream_t st)
 {
@@ -417,32 +388,32 @@ static void launch_step_lanes(const Params &p, cudaStream_t st, bool part)
     switch (p.step_lanes)
     {
     case 2:
-        BS_STEP_LAUNCH(k_step<MODE, SM, 2, false>, nb, kStepKernelBlock, 0, st, p);
+        launch_plain(k_step<MODE, SM, 2, false>, nb, kStepKernelBlock, 0, st, p);
         break;
     case 8:
         if (lean)
-            BS_STEP_LAUNCH(k_step<MODE, SM, 8, true>, nb, kStepKernelBlock, 0, st, p);
+            launch_plain(k_step<MODE, SM, 8, true>, nb, kStepKernelBlock, 0, st, p);
         else
-            BS_STEP_LAUNCH(k_step<MODE, SM, 8, false>, nb, kStepKernelBlock, 0, st, p);
+            launch_plain(k_step<MODE, SM, 8, false>, nb, kStepKernelBlock, 0, st, p);
         break;
     case 16:
         if (lean)
-            BS_STEP_LAUNCH(k_step<MODE, SM, 16, true>, nb, kStepKernelBlock, 0, st, p);
+            launch_plain(k_step<MODE, SM, 16, true>, nb, kStepKernelBlock, 0, st, p);
         else
-            BS_STEP_LAUNCH(k_step<MODE, SM, 16, false>, nb, kStepKernelBlock, 0, st, p);
+            launch_plain(k_step<MODE, SM, 16, false>, nb, kStepKernelBlock, 0, st, p);
         break;
     default:
         // without the energy sums a smaller block costs nothing and ends its wave earlier (256 -> 128 threads:
         // calls of 20 steps at 100,000 particles 1,564 -> 1,557 us, of 10 at 300,007 2,390 -> 2,356 us; 64
         // threads 1,601 and 2,353)
         if (MODE == MODE_STEP && part && lean)
-            BS_STEP_LAUNCH(k_step<MODE_STEP_PART, SM, 4, true>, np, kStepPartBlock, 0, st, p);
+            launch_plain(k_step<MODE_STEP_PART, SM, 4, true>, np, kStepPartBlock, 0, st, p);
         else if (MODE == MODE_STEP && part)
-            BS_STEP_LAUNCH(k_step<MODE_STEP_PART, SM, 4, false>, np, kStepPartBlock, 0, st, p);
+            launch_plain(k_step<MODE_STEP_PART, SM, 4, false>, np, kStepPartBlock, 0, st, p);
         else if (lean)
-            BS_STEP_LAUNCH(k_step<MODE, SM, 4, true>, nb, kStepKernelBlock, 0, st, p);
+            launch_plain(k_step<MODE, SM, 4, true>, nb, kStepKernelBlock, 0, st, p);
         else
-            BS_STEP_LAUNCH(k_step<MODE, SM, 4, false>, nb, kStepKernelBlock, 0, st, p);
+            launch_plain(k_step<MODE, SM, 4, false>, nb, kStepKernelBlock, 0, st, p);
         break;
     }
 }
@@ -590,13 +561,13 @@ int launch_step(const Params &p, int mode, cudaStream_t st)
         launched += launch_rigid(p, st); // after the step kernel, on the same stream
     if (mode != MODE_FORCES && p.probe_on)
     {
-        BS_STEP_LAUNCH(k_probe, 1, 1024, 0, st, p);
+        launch_plain(k_probe, 1, 1024, 0, st, p);
         launched += 1;
     }
     if (mode != MODE_FORCES && p.frame_every > 0)
     {
-        BS_STEP_LAUNCH(k_frame_open, 1, 1, 0, st, p);
-        BS_STEP_LAUNCH(k_frame, std::min((p.n + 255) / 256, 608), 256, 0, st, p);
+        launch_plain(k_frame_open, 1, 1, 0, st, p);
+        launch_plain(k_frame, std::min((p.n + 255) / 256, 608), 256, 0, st, p);
         launched += 2;
     }
     return launched;
@@ -634,6 +605,12 @@ int launch_step_only(const Params &p, int mode, cudaStream_t st)
     }
 #undef BS_STEP_CASE
     return 1;
+}
+
+cudaError_t load_step_kernels()
+{
+    cudaFuncAttributes a;
+    return cudaFuncGetAttributes(&a, k_unsort);
 }
 
 int launch_unsort(const Params &p, int what, float *out3, cudaStream_t st)

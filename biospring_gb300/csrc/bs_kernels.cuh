@@ -18,24 +18,22 @@ constexpr int kStepBlock = 128; // adjoint and diagnostic kernels
 constexpr int kStepKernelBlock = BS_STEP_BLOCK;
 constexpr int kStepMinBlocks = BS_STEP_MIN_BLOCKS;
 constexpr int kStepPartBlock = 128; // of the steps whose energies are not summed
-constexpr int kBuildBlock = 128;
 constexpr int kBuildLanes = 8;    // threads per slot of the spring-table rebuild when the table fits L2
 // k_order: most blocks of its grid, and the threads a particle it is sized for (small systems use as few
 // blocks as their spring table needs, for cheaper barriers)
 constexpr int kOrderMaxBlocks = 1024;
 constexpr int kOrderLanes = 8;
-constexpr int kMaxEnergyBlocks = 1 << 16;
 
 // status bits that stop a rebuild; a stale list is what a rebuild repairs
 constexpr int kRebuildBlocking = ST_NONFINITE | ST_PAIR_CAPACITY | ST_CELL_CAPACITY | ST_WIDE | ST_BARRIER;
-// Programmatic dependent launch in the rebuild chain (its eleven kernels overlap their launches:
-// 351 -> 344 us at 100k). BS_PDL_STEP extends it to the step kernels, which made the graph-replayed
-// 100k step slower (120 -> 130 us), so it is off.
 // Coulomb rows walked by the whole warp, one charged particle at a time, instead of by the
 // particle's own lanes (100k step after an L2 flush: 112.0 -> 110.8 us; warm: unchanged).
 #ifndef BS_COUL_WARP
 #define BS_COUL_WARP 1
 #endif
+// Programmatic dependent launch: the list builds begin launching while k_order runs. Step kernels keep full
+// stream ordering: launched early they take the slots of the step before them (calls of 20 steps at
+// 100,000 particles 1,557 -> 1,768 us with the trigger at their start, 1,591 us with it at their end).
 #ifndef BS_PDL
 #define BS_PDL 1
 #endif
@@ -64,19 +62,12 @@ constexpr int kGatherU = 4;
 #ifndef BS_LEAN
 #define BS_LEAN 1
 #endif
-#ifndef BS_PDL_STEP
-#define BS_PDL_STEP 0
-#endif
-// Cell-block list build on cells of half the list radius, in groups of 2 x 2 x 2 cells per block,
-// the bounded runs packed into full windows and spring partners excluded by lane masks: 323
-// candidates tested per particle instead of 505 at 100k (rebuild 355 -> 310 us).
+// Dense list build: cells of half the list radius, in groups of 2 x 2 x 2 cells per block (bs_list.cu).
 #ifndef BS_GRID_DIV
 #define BS_GRID_DIV 2
 #endif
 constexpr int kGridDiv = BS_GRID_DIV; // cell-block list build: cells per list radius (stencil of +-kGridDiv cells)
 constexpr int kSparseDiv = 1;         // warp-per-particle list build (sparse systems, batches): cells of the radius
-constexpr int kPlBatch = 16;         // home particles per warp
-constexpr int kPlBatchesPerCell = 4; // warps per cell (a cell with more than 64 particles loops)
 
 enum StepMode
 {
@@ -104,6 +95,11 @@ cudaError_t launch_run(const Params &p, int count, cudaStream_t stream, float4 *
                        float4 *save_lo = nullptr);
 cudaError_t run_fits(Params &p); // sets run_on and run_hold
 int run_blocks(const Params &p);
+// the kernel for a steric form (null where there is none for these lanes and this hold)
+const void *run_linear(int lanes, bool lean, int hold);
+const void *run_amber(int lanes, bool lean, int hold);
+const void *run_lewitt(int lanes, bool lean, int hold);
+const void *run_zacharias(int lanes, bool lean, int hold);
 // Steps of one launch (10 in the default schedule) and the polls after which a barrier gives up (some
 // seconds; a meeting takes about a microsecond).
 constexpr int kRunMaxSteps = 1024;
@@ -120,6 +116,9 @@ int launch_set_burying(const Params &p, const float *burying, cudaStream_t strea
 int launch_set_charges(const Params &p, const float *q, cudaStream_t st);
 // new stiffness and rest length (nullable, by spring) into the nnz entries of the caller-order spring table
 int launch_set_springs(const Params &p, int nnz, const unsigned int *sid, const float *k, const float *r0, cudaStream_t st);
+// Loads the module of the step and state kernels (9 ms, once a process), which is otherwise loaded by the first
+// launch of one of them: a getter, for a small system. Called at set-up.
+cudaError_t load_step_kernels();
 int launch_unsort(const Params &p, int what, float *out3, cudaStream_t stream);
 int launch_diag_cells(const Params &p, float cutoff, float skin, uint32_t need_flag, long long *out,
                       cudaStream_t stream);

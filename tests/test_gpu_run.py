@@ -1,6 +1,6 @@
 """The kernel of several steps (one cooperative launch between two list rebuilds) against the same steps
 launched one kernel at a time: positions, velocities, energies and the step count bit for bit, at the
-edges of its blocks and of its range (16 lanes a particle below 8,000, 8 below 20,000, 4 up to the 38,912
+edges of its blocks and of its range (16 lanes a particle below 8,000, 8 up to 19,456, 4 up to the 38,912
 that 608 resident blocks hold; rows held in registers up to 4,864 and 7,296 with 16 lanes, 14,592 with 8), across stale lists and with bodies. With the probe, whose reaction is summed
 in another order (float-float, then rounded once), positions agree to 1e-6 A."""
 
