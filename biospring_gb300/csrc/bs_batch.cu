@@ -531,7 +531,9 @@ __global__ void __launch_bounds__(kBatchMaxBlock, 2) k_batch_run(Params p, int c
         float e[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         const int span = (n1 - n0) * T;
         bool stop = dead; // the same in every thread of the group
-        while (!stop && !failed && done + k < upto)
+        // (a system far behind takes its steps in several launches, so that the barrier word cannot overflow)
+        const long long last = min(upto, done + max(chunk, kBatchCatchUp));
+        while (!stop && !failed && done + k < last)
         {
             const int sb = sb0 ^ (k & 1);
 #pragma unroll

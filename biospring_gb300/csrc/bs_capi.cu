@@ -508,7 +508,7 @@ int assign_clusters(bs_sim *s)
     // the barrier word of a group counts 2^30 arrivals a launch: two a system and one a step
     for (int c = 0; c < ncl; ++c)
     {
-        const double meetings = static_cast<double>(lists[c].size()) * (std::max(1, s->cfg.rebuild_every) + 4.0);
+        const double meetings = static_cast<double>(lists[c].size()) * (std::max(kBatchCatchUp, s->cfg.rebuild_every) + 4.0);
         if (meetings * size[c] > 1.0e9)
         {
             used -= size[c] - 1;

@@ -164,5 +164,6 @@ cudaError_t launch_batch_run(const Params &p, const BatchShape &shape, int chunk
 int launch_batch_finish(const Params &p, int chunk, cudaStream_t stream);
 cudaError_t batch_max_blocks(const Params &p, const BatchShape &shape, int *out); // resident at once
 constexpr int kBatchMaxBlocks = 4096; // of a launch
+constexpr int kBatchCatchUp = 65536;  // steps of one system in a launch, or the launch's own if those are more
 
 } // namespace bsg

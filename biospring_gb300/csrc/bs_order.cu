@@ -295,8 +295,15 @@ __global__ void __launch_bounds__(kOrderBlock, 4) k_order(Params p)
             float edge = p.list_radius / static_cast<float>(p.pl_sparse ? kSparseDiv : kGridDiv);
             int dims[3];
             double gmin[3];
-            const double cells = p.lists_off ? free_grid_dims(mn, mx, edge, free_cells(p.n), gmin, dims)
-                                             : grid_dims(mn, mx, edge, gmin, dims);
+            double cells = p.lists_off ? free_grid_dims(mn, mx, edge, free_cells(p.n), gmin, dims)
+                                       : grid_dims(mn, mx, edge, gmin, dims);
+            if (!(mn[0] <= mx[0] && mn[1] <= mx[1] && mn[2] <= mx[2]))
+            {
+                // no particle has a coordinate: one cell for all, the step reports them
+                dims[0] = dims[1] = dims[2] = 1;
+                gmin[0] = gmin[1] = gmin[2] = 0.0;
+                cells = 1.0;
+            }
             for (int k = 0; k < 3; ++k)
                 sh_grid.gmin[k] = gmin[k];
             sh_grid.radius = edge;

@@ -9,6 +9,7 @@ from __future__ import annotations
 import numpy as np
 import pytest
 
+from biospring_gb300 import BsError
 from biospring_gb300 import workloads as W
 from helpers import gpu_network, load_golden, system_from_golden
 
@@ -71,6 +72,18 @@ def test_stale_list_stops_and_resumes():
     for _ in range(37):
         b.computeStep(1)
     _same(a, b, 37)
+
+
+@pytest.mark.parametrize("axes", [(0,), (0, 1, 2)])
+def test_no_coordinates_are_reported(axes):
+    s = _system(300)
+    net = gpu_network(s)
+    x = s.xyz.copy()
+    x[:, list(axes)] = np.nan
+    net.setPositions(x)
+    with pytest.raises(BsError):
+        net.computeStep(2)
+    net.close()
 
 
 def test_external_force_acts_on_the_first_step():
