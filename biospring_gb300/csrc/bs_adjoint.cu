@@ -215,10 +215,15 @@ __device__ __forceinline__ float4 adj_update(const Params &p, float m, float hx,
 // One backward step for every particle: reads nu of step n+1 and the positions at the start of
 // step n, updates lambda_x and lambda_v in place, writes nu of step n, and adds this step's
 // terms to the per-entry spring gradients. T lanes per particle, as in the forward step.
+// A rebuild that was blocked (a grid or list too small, offsets that left 16 bits) leaves the spring ids and
+// the lists of another layout or cut short: the backward steps behind it do nothing, and the host grows what was too
+// small and runs everything again.
 template <int T>
 __global__ void __launch_bounds__(kStepBlock) k_adj_step(Params p, AdjState a)
 {
     const Ctl *ctl = p.ctl;
+    if (status_of(ctl) & kRebuildBlocking)
+        return;
     const int lb = ctl->lbuf;
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     const int s = g / T, t = g % T;
@@ -297,6 +302,8 @@ template <int T>
 __global__ void __launch_bounds__(kAdjRunBlock, T == 4 ? 3 : 2) k_adj_run(Params p, AdjState a, int count)
 {
     const Ctl *ctl = p.ctl;
+    if (status_of(ctl) & kRebuildBlocking)
+        return; // the same in every block: only a timed-out barrier raises such a bit in this kernel
     const int lb = ctl->lbuf;
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     const int s = g / T, t = g % T;

@@ -2532,6 +2532,7 @@ int bs_adjoint(bs_sim *s, int32_t nsteps, int32_t checkpoint, const float *targe
             return rc;
         unsigned int *e_sid = nullptr;
         BS_CUDA(s->adj_dev.alloc(&e_sid, np * p.sp_maxdeg));
+        BS_CUDA(cudaMemsetAsync(e_sid, 0, sizeof(unsigned int) * np * p.sp_maxdeg, s->stream));
         p.sp_sid = s->sp_sid_d;
         p.se_sid = e_sid;
         destroy_graph(s);
