@@ -409,21 +409,56 @@ int rebuild_now(bs_sim *s)
     return fail(s, BS_E_CAPACITY, "pair list or grid did not fit after repeated growth");
 }
 
+// After launches on the handle's stream: if one was refused, the rebuild may be the one that is missing.
+int check_launches(bs_sim *s)
+{
+    const cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess)
+        return BS_OK;
+    s->list_valid = false;
+    return cuda_fail(s, e, "kernel launch");
+}
+
+// Recording of a graph on the handle's stream. A launch that is refused while it is recorded is missing from the
+// graph, and some launchers leave that to the thread's last error alone, so it is read before the graph is kept.
+int begin_graph(bs_sim *s)
+{
+    cudaGetLastError(); // what an earlier call of the thread left is not this recording's
+    BS_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
+    return BS_OK;
+}
+
+int end_graph(bs_sim *s, cudaGraphExec_t *graph, int rc, const char *what)
+{
+    cudaGraph_t g = nullptr;
+    const cudaError_t launched = cudaGetLastError();
+    cudaError_t e = cudaStreamEndCapture(s->stream, &g);
+    if (rc == BS_OK && launched == cudaSuccess && e == cudaSuccess)
+        e = cudaGraphInstantiate(graph, g, 0);
+    if (g)
+        cudaGraphDestroy(g);
+    if (rc != BS_OK)
+        return rc;
+    if (launched != cudaSuccess)
+        e = launched;
+    if (e == cudaSuccess)
+        return BS_OK;
+    *graph = nullptr;
+    return cuda_fail(s, e, what);
+}
+
 int capture_period_graph(bs_sim *s)
 {
     destroy_graph(s);
     const int K = std::max(1, s->cfg.rebuild_every);
-    cudaGraph_t g = nullptr;
-    BS_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
+    int rc = begin_graph(s);
+    if (rc)
+        return rc;
     int kernels = launch_rebuild(s->p, s->stream);
     kernels += launch_steps(s->p, K, s->stream);
-    BS_CUDA(cudaStreamEndCapture(s->stream, &g));
-    const cudaError_t e = cudaGraphInstantiate(&s->period_graph, g, 0);
-    cudaGraphDestroy(g);
-    if (e != cudaSuccess)
-        return cuda_fail(s, e, "cudaGraphInstantiate");
+    rc = end_graph(s, &s->period_graph, BS_OK, "recording a period of steps");
     s->period_kernels = kernels;
-    return BS_OK;
+    return rc;
 }
 
 // Assigns whole systems to the block groups of the persistent batched kernel: as many groups as the
@@ -537,26 +572,16 @@ int capture_batch_graph(bs_sim *s)
 {
     destroy_graph(s);
     const int K = std::max(1, s->cfg.rebuild_every);
-    cudaGraph_t g = nullptr;
-    BS_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
+    int rc = begin_graph(s);
+    if (rc)
+        return rc;
     int kernels = launch_rebuild(s->p, s->stream);
     const cudaError_t le = launch_batch_run(s->p, s->shape, K, s->stream);
     kernels += 1 + launch_batch_finish(s->p, K, s->stream);
-    const cudaError_t ce = cudaStreamEndCapture(s->stream, &g);
-    if (le != cudaSuccess)
-    {
-        if (g)
-            cudaGraphDestroy(g);
-        return cuda_fail(s, le, "batched step launch");
-    }
-    if (ce != cudaSuccess)
-        return cuda_fail(s, ce, "cudaStreamEndCapture");
-    const cudaError_t e = cudaGraphInstantiate(&s->period_graph, g, 0);
-    cudaGraphDestroy(g);
-    if (e != cudaSuccess)
-        return cuda_fail(s, e, "cudaGraphInstantiate");
+    rc = end_graph(s, &s->period_graph, le == cudaSuccess ? BS_OK : cuda_fail(s, le, "batched step launch"),
+                   "recording a period of ensemble steps");
     s->period_kernels = kernels;
-    return BS_OK;
+    return rc;
 }
 
 // Enqueues `count` nominal steps of a batched ensemble on the rebuild schedule of the single-system
@@ -601,8 +626,7 @@ int enqueue_batch(bs_sim *s, long long count, bool catchup)
         s->since_rebuild += chunk;
         remaining -= chunk;
     }
-    BS_CUDA(cudaGetLastError());
-    return BS_OK;
+    return check_launches(s);
 }
 
 // The double membrane into the step parameters (flat when every value is zero).
@@ -1657,8 +1681,7 @@ static int enqueue_steps(bs_sim *s, long long count)
         s->since_rebuild += static_cast<int>(chunk);
         remaining -= chunk;
     }
-    BS_CUDA(cudaGetLastError());
-    return BS_OK;
+    return check_launches(s);
 }
 
 int bs_step_async(bs_sim *s, int32_t nsteps)
@@ -1809,8 +1832,7 @@ int bs_launch_phase(bs_sim *s, int32_t phase)
     }
     else
         return fail(s, BS_E_ARG, "bs_launch_phase: phase must be 0 or 1");
-    BS_CUDA(cudaGetLastError());
-    return BS_OK;
+    return check_launches(s);
 }
 
 static int set_external_forces(bs_sim *s, const float *f, bool wait);
@@ -2580,27 +2602,21 @@ int bs_adjoint(bs_sim *s, int32_t nsteps, int32_t checkpoint, const float *targe
                 cudaGraphExecDestroy(s->adj_graph);
                 s->adj_graph = nullptr;
             }
-            cudaGraph_t g = nullptr;
-            BS_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
+            rc = begin_graph(s);
+            if (rc)
+                return rc;
             const long long before = s->launches;
             // the adjoint's forward runs record no frames
             const int frame_every = s->p.frame_every;
             s->p.frame_every = 0;
             rc = record_adjoint(s, nsteps, K, charges, keep_all);
             s->p.frame_every = frame_every;
-            const cudaError_t ce = cudaStreamEndCapture(s->stream, &g);
+            rc = end_graph(s, &s->adj_graph, rc, "bs_adjoint: recording the run");
             if (rc)
             {
-                if (g)
-                    cudaGraphDestroy(g);
+                s->launches = before;
                 return rc;
             }
-            if (ce != cudaSuccess)
-                return cuda_fail(s, ce, "bs_adjoint: capture");
-            const cudaError_t ie = cudaGraphInstantiate(&s->adj_graph, g, 0);
-            cudaGraphDestroy(g);
-            if (ie != cudaSuccess)
-                return cuda_fail(s, ie, "bs_adjoint: cudaGraphInstantiate");
             s->adj_key[0] = nsteps;
             s->adj_key[1] = K;
             s->adj_key[2] = charges ? 1 : 0;
