@@ -25,6 +25,8 @@
 // 100,000 particles 234 -> 145, 12,000 71 -> 44, 6,007 with three radii 50 -> 36. The rows by one warp a home,
 // a word or an output window at a time, took 159; one or two threads a home 171 and 157.
 
+#include <algorithm>
+
 #include "bs_device.cuh"
 
 namespace bsg
@@ -35,6 +37,8 @@ namespace
 constexpr int kListWarps = 8;
 constexpr int kListThreads = 32 * kListWarps;
 constexpr int kListBlocks = 5;                  // resident blocks per SM
+constexpr int kListResident = 152 * kListBlocks;
+constexpr int kListFull = 152 * 4;              // blocks that fill the chip
 constexpr int kListTile = 1536;                 // candidates staged at once
 constexpr int kListChunks = kListTile / 32;
 constexpr int kListHomes = 64;                  // homes of a batch
@@ -224,9 +228,10 @@ template <bool PL16, int SPLIT> __global__ void __launch_bounds__(kListThreads, 
     unsigned int held[kHeld] = {};
     constexpr int E = 4 * SPLIT, kHomes = kListThreads / E;    // threads a home; homes of a batch
     const int hq = threadIdx.x / E, tq = threadIdx.x % E; // this thread's home of the batch, and which of its threads it is
-    for (int item = blockIdx.x; item < ngroups * SPLIT; item += gridDim.x)
+    const bool whole = SPLIT == 1 || (ngroups >= kListFull && 24ll * ngroups > p.n);
+    for (int item = blockIdx.x; item < (whole ? ngroups : ngroups * SPLIT); item += gridDim.x)
     {
-        const int grp = item / SPLIT, part = item % SPLIT;
+        const int grp = whole ? item : item / SPLIT, part = item % SPLIT;
         const int gx0 = grp % ngx * kG, gy0 = grp / ngx % ngy * kG, gz0 = grp / (ngx * ngy) * kG;
         const int xa = max(gx0 - kD, 0), xb = min(gx0 + kG - 1 + kD, nx - 1), hxb = min(gx0 + kG - 1, nx - 1);
         __syncthreads(); // the previous group's tables are no longer read
@@ -313,7 +318,8 @@ template <bool PL16, int SPLIT> __global__ void __launch_bounds__(kListThreads, 
             }
         }
         __syncthreads();
-        const int n_cand = sh_off[kRows], h0 = n_home * part / SPLIT, h1 = n_home * (part + 1) / SPLIT;
+        const int n_cand = sh_off[kRows];
+        const int h0 = whole ? 0 : n_home * part / SPLIT, h1 = whole ? n_home : n_home * (part + 1) / SPLIT;
         for (int hb = h0; hb < h1; hb += kHomes)
         {
             const int nhb = min(kHomes, h1 - hb);
@@ -491,10 +497,13 @@ template <bool PL16, int SPLIT> __global__ void __launch_bounds__(kListThreads, 
 
 template <int SPLIT> static void launch_split(const Params &p, cudaStream_t st)
 {
-    // the number of groups is only known on the device: cover the capacity (blocks past the last return at
-    // once, and the kernel strides over what is left)
+    // The number of groups is only known on the device. A dense system (8 particles a group and more) has n / 8 at
+    // most, or no more than the capacity: that many blocks, of which those past the last group return at once. One that
+    // has spread out since has more, mostly empty ones: the blocks stride over them (12,000 particles eight times as far
+    // apart, a block for each part of a group: 1,233 us a rebuild; so 246).
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(static_cast<unsigned>(SPLIT * (p.cell_cap / (kGridDiv * kGridDiv * kGridDiv) + 1)));
+    const int groups = std::min(p.cell_cap / (kGridDiv * kGridDiv * kGridDiv) + 1, std::max(p.n / 8, kListResident));
+    cfg.gridDim = dim3(static_cast<unsigned>(SPLIT * groups));
     cfg.blockDim = dim3(kListThreads);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -510,7 +519,10 @@ template <int SPLIT> static void launch_split(const Params &p, cudaStream_t st)
 
 // A group's homes are split over 4 blocks up to 16,384 particles and over 2 up to 32,768: a block a
 // group left half the SMs with one block or none at 6,000 particles. Measured (ncu, us a build, whole groups
-// against split): 6,007 particles 57 -> 39, 12,000 46 -> 46 (2 parts 48).
+// against split): 6,007 particles 57 -> 39, 12,000 46 -> 46 (2 parts 48). Where the particles have spread out, so that the
+// groups alone fill the chip and hold fewer than 24 homes each, a block takes a whole group (us a rebuild, split against
+// whole: 16,000 particles at 0.0244 per cubic A 1.4 times as far apart 86 -> 67, 1.7 times 98 -> 63; 24 homes are where the
+// two meet: 1.2 times as far apart, 22 homes, 81 and 80).
 int launch_pairlist(const Params &p, cudaStream_t st)
 {
     if (p.n <= 16384)
