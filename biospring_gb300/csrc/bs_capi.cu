@@ -23,9 +23,15 @@ namespace
 
 thread_local std::string g_last_error;
 
-// Largest result a kernel writes straight into page-locked host memory; beyond, a copy engine's transfer
-// of the whole array is the faster way out.
-constexpr size_t kDirectOut = 256 * 1024;
+// Largest result a kernel writes straight into page-locked host memory; beyond, a copy of the whole array is the
+// faster way out. Measured (us a getPositions, direct and by copy): 300 particles 24 and 26, 2,000 26 and 26, 4,000 28
+// and 27, 8,000 33 and 27, 20,000 52 and 28.
+constexpr size_t kDirectOut = 24 * 1024;
+// Largest pageable state (positions, velocities) that goes in through the handle's pinned buffer; beyond, one
+// thread's copy into that buffer is slower than the transfer straight out of the caller's pages. Measured (us a
+// setPositions, staged and straight): 300 particles 21 and 24, 8,000 21 and 32, 30,000 31 and 33, 50,000 43 and 36,
+// 1,000,000 812 and 112.
+constexpr size_t kStagedIn = 384 * 1024;
 
 struct DeviceBuffers
 {
@@ -260,18 +266,18 @@ cudaMemoryType memory_type(const void *p)
     return cudaMemoryTypeUnregistered;
 }
 
-// Enqueues a copy of up to 3n floats of the caller's to the device. A pageable source goes through the
-// handle's pinned buffer, so the caller may reuse it when this returns and the call waits for nothing but an
-// earlier copy out of that buffer; any other must stay unchanged until the stream is waited for.
-int upload(bs_sim *s, float *dst, const float *src, size_t floats, bool pinned)
+// Enqueues a copy of up to 3n floats of the caller's to the device: through the handle's pinned buffer, so that the
+// caller may reuse a pageable source when this returns and the call waits for nothing but an earlier copy out of that
+// buffer, or straight from the source, which must then stay unchanged until the stream is waited for.
+int upload(bs_sim *s, float *dst, const float *src, size_t floats, bool straight)
 {
-    if (!pinned)
+    if (!straight)
     {
         BS_CUDA(cudaEventSynchronize(s->stage_event));
         std::memcpy(s->stage_h, src, floats * sizeof(float));
     }
-    BS_CUDA(cudaMemcpyAsync(dst, pinned ? src : s->stage_h, floats * sizeof(float), cudaMemcpyHostToDevice, s->stream));
-    if (!pinned)
+    BS_CUDA(cudaMemcpyAsync(dst, straight ? src : s->stage_h, floats * sizeof(float), cudaMemcpyHostToDevice, s->stream));
+    if (!straight)
         BS_CUDA(cudaEventRecord(s->stage_event, s->stream));
     return BS_OK;
 }
@@ -1957,13 +1963,14 @@ static int set_state(bs_sim *s, const float *xyz, const float *vel)
     int rc = settle(s);
     if (rc)
         return rc;
-    const bool pinned = memory_type(src) != cudaMemoryTypeUnregistered;
-    rc = upload(s, s->staging, src, 3 * static_cast<size_t>(s->n), pinned);
+    const size_t floats = 3 * static_cast<size_t>(s->n);
+    const bool straight = floats * sizeof(float) > kStagedIn || memory_type(src) != cudaMemoryTypeUnregistered;
+    rc = upload(s, s->staging, src, floats, straight);
     if (rc)
         return rc;
     s->launches += launch_set_positions(s->p, xyz ? s->staging : nullptr, xyz ? nullptr : s->staging, s->stream);
     BS_CUDA(cudaGetLastError());
-    if (pinned)
+    if (straight)
         BS_CUDA(cudaStreamSynchronize(s->stream));
     if (xyz)
         s->list_valid = false;
