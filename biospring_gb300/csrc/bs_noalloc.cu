@@ -381,18 +381,26 @@ __global__ void __launch_bounds__(kNaBlock, 3) k_na_forces(NaParams p, int split
                 evaluate(r, f >> 16, f & 0xffffu);
         }
     }
-#pragma unroll 1
-    for (int r = 0; r < R; ++r)
+    // The lanes' sums of every home and term: at each distance a lane passes on the half of its values that the
+    // other keeps, so the values halve with the distance and lane 6 r + q ends with sum q of home r. The sums are those
+    // of a shuffle tree a value, bit for bit, with 31 shuffles instead of 120
+    // (us a call, before and now: 1 particle 12.4 and 10.4, 200 16.6 and 14.6, 4,001 49.8 and 43.8).
+    {
+        float v[32];
 #pragma unroll
-        for (int q = 0; q < NV; ++q)
-        {
-            float v = sh_acc[warp][r][q][lane];
+        for (int k = 0; k < 32; ++k)
+            v[k] = k < R * NV ? sh_acc[warp][k / NV][k % NV][lane] : 0.0f;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-                v += __shfl_down_sync(0xffffffffu, v, o);
-            if (lane == 0)
-                sh_sum[warp][r][q] = v;
-        }
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int k = 0; k < o; ++k)
+            {
+                const float keep = (lane & o) ? v[k + o] : v[k], pass = (lane & o) ? v[k] : v[k + o];
+                v[k] = keep + __shfl_xor_sync(0xffffffffu, pass, o);
+            }
+        if (lane < R * NV)
+            sh_sum[warp][lane / NV][lane % NV] = v[0];
+    }
     __syncthreads();
     // one thread a home adds the split warps' sums; energies go on in FP64, home by home
     if (part == 0 && lane < R)
