@@ -24,9 +24,9 @@ namespace
 thread_local std::string g_last_error;
 
 // Largest result a kernel writes straight into page-locked host memory; beyond, a copy of the whole array is the
-// faster way out. Measured (us a getPositions, direct and by copy): 300 particles 24 and 26, 2,000 26 and 26, 4,000 28
-// and 27, 8,000 33 and 27, 20,000 52 and 28.
-constexpr size_t kDirectOut = 24 * 1024;
+// faster way out. Measured (us a getPositions, direct and by copy): a chain of 2,217 particles 24 and 27, 3,700 26 and
+// 27, 6,000 28 and 27, 12,000 34 and 28; in random order 2,000 26 and 26, 4,000 28 and 27, 8,000 33 and 27, 20,000 52 and 28.
+constexpr size_t kDirectOut = 48 * 1024;
 // Largest pageable state (positions, velocities) that goes in through the handle's pinned buffer; beyond, one
 // thread's copy into that buffer is slower than the transfer straight out of the caller's pages. Measured (us a
 // setPositions, staged and straight): 300 particles 21 and 24, 8,000 21 and 32, 30,000 31 and 33, 50,000 43 and 36,

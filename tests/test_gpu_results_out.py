@@ -1,4 +1,4 @@
-"""Results on both sides of the 24 KB (2,048 particles) up to which the kernel writes them to the host itself, and
+"""Results on both sides of the 48 KB (4,096 particles) up to which the kernel writes them to the host itself, and
 states on both sides of the 384 KB (32,768 particles) up to which they go in through the handle's own buffer, one after
 the other. All bit for bit."""
 
@@ -13,7 +13,7 @@ from helpers import gpu_network
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [2048, 2049, 32768, 32769])
+@pytest.mark.parametrize("n", [2048, 2049, 4096, 4097, 32768, 32769])
 def test_states_in_and_results_out(n):
     rng = np.random.default_rng(n)
     a, b, v = (rng.uniform(0.0, 3.0 * n ** (1 / 3), (n, 3)).astype(np.float32) for _ in range(3))
