@@ -133,6 +133,11 @@ __device__ __forceinline__ double free_grid_dims(const float (&mn)[3], const flo
     return cells;
 }
 
+// Every product that meets a sum is rounded or fused here as written, not as the compiler sees fit: it decides by what
+// else an instance computes, and a step must give the same bits in every kernel and form that takes it (alone, in
+// k_run with rows held or not, without its energies).
+__device__ __forceinline__ float norm2(float x, float y, float z) { return fmaf(z, z, fmaf(x, x, y * y)); }
+
 // Exact reference test of one candidate pair for one cutoff: the grid filter compares the FP64
 // distance of the float coordinates (nsearch.hpp:230, measure.hpp:163-169); the force routine
 // then compares the float-rounded FP64 norm of the float difference vector (Particle.cpp:222-224,
@@ -413,10 +418,9 @@ __device__ __forceinline__ void spring_forces(const Params &p, int s, int t, flo
         if (c & kEntryInactive)
             continue;
         const float dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
-        const float r2 = dx * dx + dy * dy + dz * dz;
+        const float r2 = norm2(dx, dy, dz);
         const float inv = r2 > 0.0f ? rsqrt_nr(r2) : 0.0f;
-        const float len = r2 * inv;
-        const float dv = len - r0;
+        const float dv = fmaf(r2, inv, -r0);
         const float w = (c & kEntryStatic) ? 1.0f : 0.5f;
         e = fmaf(w * 0.5f * kk, dv * dv, e);
         const float fod = kk * dv * inv;
@@ -424,6 +428,39 @@ __device__ __forceinline__ void spring_forces(const Params &p, int s, int t, flo
         fy = fmaf(dy, fod, fy);
         fz = fmaf(dz, fod, fz);
     }
+}
+
+// The LJ pair body: adds the pair's weighted energy to e and returns the force over distance (both zero for a
+// rejected pair). ok says whether the pair is in the cutoff. STATIC, a static partner: the Amber form fuses the
+// repulsive product with its difference, otherwise the products are rounded first.
+template <int SM, bool STATIC = false>
+__device__ __forceinline__ float lj_pair(float r2, bool ok, float pw, float fhi_i, float4 pj, float hj, float w,
+                                         float &e)
+{
+    const float inv2 = recip_lj(r2);
+    const float i6 = inv2 * inv2 * inv2;
+    const float t6 = __fmul_rn(pw * pj.w, i6);
+    float fod, de;
+    if (SM == BS_STERIC_LJ_12_6_AMBER)
+    {
+        const float a = fhi_i * hj * i6, t12 = __fmul_rn(a, i6);
+        de = STATIC ? fmaf(a, i6, -2.0f * t6) : fmaf(-2.0f, t6, t12);
+        fod = 12.0f * (STATIC ? fmaf(-a, i6, t6) : t6 - t12) * inv2;
+    }
+    else if (SM == BS_STERIC_LJ_8_6_LEWITT)
+    {
+        const float t8 = __fmul_rn(fhi_i * hj * i6, inv2);
+        de = fmaf(3.0f, t8, -4.0f * t6);
+        fod = 24.0f * (t6 - t8) * inv2;
+    }
+    else
+    {
+        const float t8 = __fmul_rn(fhi_i * hj * i6, inv2);
+        de = t8 - t6;
+        fod = fmaf(6.0f, t6, -8.0f * t8) * inv2;
+    }
+    e = fmaf(w, ok ? de : 0.0f, e);
+    return ok ? fod : 0.0f;
 }
 
 // Steric pairs of slot s handled by lane t of T (Particle.cpp:368-429, steric.hpp:27-156).
@@ -469,7 +506,7 @@ __device__ __forceinline__ void steric_forces(const Params &p, int s, int t, flo
                 hn = __ldg(&fhi[jn]);
         }
         const float dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
-        const float r2 = dx * dx + dy * dy + dz * dz;
+        const float r2 = norm2(dx, dy, dz);
         if (SM == BS_STERIC_LINEAR)
         {
             // Few listed pairs overlap: the branches skip the square root and division of the rest.
@@ -500,69 +537,12 @@ __device__ __forceinline__ void steric_forces(const Params &p, int s, int t, flo
             if (!ok && r2 < hi2)
                 ok = exact_pair_test(pi, pj, p.c_steric, false);
             ok = ok && !(r2 < 0.01f); // d < 0.1 A: the LJ forms give zero (steric.hpp:71-72)
-            const float inv2 = recip_nr(r2);
-            const float i6 = inv2 * inv2 * inv2;
-            const float t6 = pi.w * pj.w * i6;
-            float fod, de;
-            if (SM == BS_STERIC_LJ_12_6_AMBER)
-            {
-                const float t12 = fhi_i * hj * i6 * i6;
-                de = t12 - 2.0f * t6;
-                fod = 12.0f * (t6 - t12) * inv2;
-            }
-            else if (SM == BS_STERIC_LJ_8_6_LEWITT)
-            {
-                const float t8 = fhi_i * hj * i6 * inv2;
-                de = 3.0f * t8 - 4.0f * t6;
-                fod = 24.0f * (t6 - t8) * inv2;
-            }
-            else
-            {
-                const float t8 = fhi_i * hj * i6 * inv2;
-                de = t8 - t6;
-                fod = (6.0f * t6 - 8.0f * t8) * inv2;
-            }
-            e = fmaf(w, ok ? de : 0.0f, e);
-            fod = ok ? fod : 0.0f;
+            const float fod = lj_pair<SM, KIND == 2>(r2, ok, pi.w, fhi_i, pj, hj, w, e);
             fx = fmaf(dx, fod, fx);
             fy = fmaf(dy, fod, fy);
             fz = fmaf(dz, fod, fz);
         }
     }
-}
-
-// The LJ pair body of steric_forces: adds the pair's weighted energy to e and returns the force
-// over distance (both zero for a rejected pair). ok says whether the pair is in the cutoff.
-template <int SM>
-__device__ __forceinline__ float lj_pair(float r2, bool ok, float pw, float fhi_i, float4 pj, float hj, float w,
-                                         float &e)
-{
-    const float inv2 = recip_lj(r2);
-    const float i6 = inv2 * inv2 * inv2;
-    // the products are rounded before the differences in every build, so that a step whose energy is not
-    // summed gives the same force bits (without it the compiler may fuse a product it uses once)
-    const float t6 = __fmul_rn(pw * pj.w, i6);
-    float fod, de;
-    if (SM == BS_STERIC_LJ_12_6_AMBER)
-    {
-        const float t12 = __fmul_rn(fhi_i * hj * i6, i6);
-        de = t12 - 2.0f * t6;
-        fod = 12.0f * (t6 - t12) * inv2;
-    }
-    else if (SM == BS_STERIC_LJ_8_6_LEWITT)
-    {
-        const float t8 = __fmul_rn(fhi_i * hj * i6, inv2);
-        de = 3.0f * t8 - 4.0f * t6;
-        fod = 24.0f * (t6 - t8) * inv2;
-    }
-    else
-    {
-        const float t8 = __fmul_rn(fhi_i * hj * i6, inv2);
-        de = t8 - t6;
-        fod = (6.0f * t6 - 8.0f * t8) * inv2;
-    }
-    e = fmaf(w, ok ? de : 0.0f, e);
-    return ok ? fod : 0.0f;
 }
 
 // Steric pairs of slot s with its dynamic partners (list 0), lane t of T, in passes of kGatherU
@@ -572,7 +552,7 @@ __device__ __forceinline__ float lj_pair(float r2, bool ok, float pw, float fhi_
 // warp waits for one round trip per U pairs instead of one per pair. Entries past the row's end
 // read the slot past the particles (far from all of them) and fail the distance test. Rows start on 16-byte boundaries (capacities are
 // multiples of 8 entries), so the vector loads are aligned and never leave the row's capacity.
-template <int SM, int T, bool PL16, bool UF, class POS>
+template <int SM, int T, bool PL16, bool UF, bool SINGLE, class POS>
 __device__ __forceinline__ void steric_forces_batched(const Params &p, int s, int t, float4 pi, float fhi_i,
                                                       const POS pos, const float *__restrict__ fhi,
                                                       float &fx, float &fy, float &fz, float &e, int cnt_in = -1,
@@ -674,7 +654,9 @@ __device__ __forceinline__ void steric_forces_batched(const Params &p, int s, in
         for (int u = 0; u < U; ++u)
         {
             const float dx = pj[u].x - pi.x, dy = pj[u].y - pi.y, dz = pj[u].z - pi.z;
-            const float r2 = dx * dx + dy * dy + dz * dz;
+            // (the ensemble kernel, of which there is one form, leaves the order to the compiler: the same bits and
+            // 20 bytes of spills less, 1,336 -> 1,331 us for 64 systems)
+            const float r2 = SINGLE ? norm2(dx, dy, dz) : dx * dx + dy * dy + dz * dz;
             if (SM == BS_STERIC_LINEAR)
             {
                 if (!(r2 < hi2))
@@ -722,7 +704,7 @@ __device__ __forceinline__ void steric_forces_batched(const Params &p, int s, in
                 if (!((band >> u) & 1u) || !exact_pair_test(pi, pj[u], p.c_steric, false))
                     continue;
                 const float dx = pj[u].x - pi.x, dy = pj[u].y - pi.y, dz = pj[u].z - pi.z;
-                const float r2 = dx * dx + dy * dy + dz * dz;
+                const float r2 = norm2(dx, dy, dz);
                 const float fod = lj_pair<SM>(r2, true, pi.w, fhi_i, pj[u], hj[u], 0.5f, e);
                 fx = fmaf(dx, fod, fx);
                 fy = fmaf(dy, fod, fy);
@@ -778,10 +760,9 @@ __device__ __forceinline__ void spring_forces_batched(const Params &p, int s, in
             if (c[u] & kEntryInactive)
                 continue;
             const float dx = pj[u].x - pi.x, dy = pj[u].y - pi.y, dz = pj[u].z - pi.z;
-            const float r2 = dx * dx + dy * dy + dz * dz;
+            const float r2 = norm2(dx, dy, dz);
             const float inv = r2 > 0.0f ? rsqrt_nr(r2) : 0.0f;
-            const float len = r2 * inv;
-            const float dv = len - r0[u];
+            const float dv = fmaf(r2, inv, -r0[u]);
             const float w = (c[u] & kEntryStatic) ? 1.0f : 0.5f;
             e = fmaf(w * 0.5f * kk[u], dv * dv, e);
             const float fod = kk[u] * dv * inv;
@@ -824,7 +805,7 @@ __device__ __forceinline__ void coulomb_forces(const Params &p, int s, int t, fl
             qn = __ldg(&chg[jn & kSlotMask]);
         }
         const float dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
-        const float r2 = dx * dx + dy * dy + dz * dz;
+        const float r2 = norm2(dx, dy, dz);
         if (!pair_in(r2, p.lo2_c, p.hi2_c, pi, pj, p.c_coulomb, true))
             continue;
         if (r2 < 1e-6f) // d < 0.001 A gives zero (electrostatic.hpp:18-19)
@@ -862,7 +843,7 @@ __device__ __forceinline__ void hydro_forces(const Params &p, int s, int t, floa
         const unsigned int j = __ldg(row + k);
         const float4 pj = pos[j & kSlotMask];
         const float dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
-        const float r2 = dx * dx + dy * dy + dz * dz;
+        const float r2 = norm2(dx, dy, dz);
         if (!pair_in(r2, p.lo2_h, p.hi2_h, pi, pj, p.c_hydro, true))
             continue;
         const float inv = rsqrt_nr(r2);
@@ -886,7 +867,7 @@ __device__ __forceinline__ void probe_pair(const Params &p, const float4 &prb, f
                                            float &fx, float &fy, float &fz, float &es, float &ec)
 {
     const float dx = prb.x - pi.x, dy = prb.y - pi.y, dz = prb.z - pi.z;
-    const float r2 = dx * dx + dy * dy + dz * dz;
+    const float r2 = norm2(dx, dy, dz);
     if (p.probe_steric)
     {
         float fod = 0.0f;
@@ -904,24 +885,24 @@ __device__ __forceinline__ void probe_pair(const Params &p, const float4 &prb, f
         {
             const float inv2 = recip_nr(r2);
             const float i6 = inv2 * inv2 * inv2;
-            const float t6 = p.probe_P * pi.w * i6;
+            const float t6 = __fmul_rn(p.probe_P * pi.w, i6);
             if (SM == BS_STERIC_LJ_12_6_AMBER)
             {
-                const float t12 = p.probe_F * fhi_i * i6 * i6;
-                es = fmaf(p.steric_scale, t12 - 2.0f * t6, es);
+                const float t12 = __fmul_rn(p.probe_F * fhi_i * i6, i6);
+                es = fmaf(p.steric_scale, fmaf(-2.0f, t6, t12), es);
                 fod = 12.0f * (t6 - t12) * inv2;
             }
             else if (SM == BS_STERIC_LJ_8_6_LEWITT)
             {
-                const float t8 = p.probe_F * fhi_i * i6 * inv2;
-                es = fmaf(p.steric_scale, 3.0f * t8 - 4.0f * t6, es);
+                const float t8 = __fmul_rn(p.probe_F * fhi_i * i6, inv2);
+                es = fmaf(p.steric_scale, fmaf(3.0f, t8, -4.0f * t6), es);
                 fod = 24.0f * (t6 - t8) * inv2;
             }
             else
             {
-                const float t8 = p.probe_F * fhi_i * i6 * inv2;
+                const float t8 = __fmul_rn(p.probe_F * fhi_i * i6, inv2);
                 es = fmaf(p.steric_scale, t8 - t6, es);
-                fod = (6.0f * t6 - 8.0f * t8) * inv2;
+                fod = fmaf(6.0f, t6, -8.0f * t8) * inv2;
             }
         }
         const float k = fod * p.k_spring_f * p.steric_scale;
@@ -1021,17 +1002,17 @@ __device__ __forceinline__ void field_forces(const Params &p, const float4 &pi, 
 __device__ __forceinline__ void imp_double_membrane(const Params &p, const float4 &pi, float S, float T, float &fx,
                                                     float &fz, float &e)
 {
-    const float gg = -S * T + kAlip * S;
+    const float gg = fmaf(kAlip, S, -__fmul_rn(S, T));
 #pragma unroll
     for (int m = 0; m < 2; ++m)
     {
         const float off = p.imp_off[m], c = p.imp_curv[m];
         const float R = c == 0.0f ? 1000000.0f : fabsf(1.0f / c);
         const float sg = c > 0.0f ? 1.0f : (c < 0.0f ? -1.0f : 0.0f);
-        const float axis = off - sg * R;
+        const float axis = fmaf(-sg, R, off);
         const float rx = pi.x, rz = pi.z - axis;
-        const float rn = sqrtf(rx * rx + rz * rz);
-        const float depth = sg == 0.0f ? pi.z : (pi.z > axis ? sg * rn : -sg * rn) + off - R;
+        const float rn = sqrtf(fmaf(rz, rz, __fmul_rn(rx, rx)));
+        const float depth = sg == 0.0f ? pi.z : fmaf(pi.z > axis ? sg : -sg, rn, off) - R;
         const float u = depth - off;
         const float ex = expf(p.imp_alpha * (fabsf(u) - p.imp_z0));
         e = fmaf(p.imp_scale * gg, 0.5f - 1.0f / (1.0f + ex), e);
@@ -1048,8 +1029,8 @@ __device__ __forceinline__ void imp_double_membrane(const Params &p, const float
             dz = rn > 1e-40f ? rz / rn : 0.0f;
         }
         const float f = p.imp_scale * (gg * dcz * p.k_imp_f);
-        fx -= f * dx;
-        fz -= f * dz;
+        fx = fmaf(-f, dx, fx);
+        fz = fmaf(-f, dz, fz);
     }
 }
 
@@ -1181,14 +1162,14 @@ __device__ __forceinline__ int particle_step(const Params &p, const int s, const
         {
             float sx = 0.f, sy = 0.f, sz = 0.f, es = 0.f;
             if (LEAN && p.lj_uniform && p.pl16)
-                steric_forces_batched<SM, T, true, true>(p, s, t, pi, fhi_i, pos, p.fhi[lb], sx, sy, sz, es, cnt0, w0);
+                steric_forces_batched<SM, T, true, true, SINGLE>(p, s, t, pi, fhi_i, pos, p.fhi[lb], sx, sy, sz, es, cnt0, w0);
             else if ((SINGLE && BS_GATHER) || (!SINGLE && BS_GATHER_BATCH))
             {
                 if (p.pl16)
-                    steric_forces_batched<SM, T, true, false>(p, s, t, pi, fhi_i, pos, p.fhi[lb], sx, sy, sz, es,
+                    steric_forces_batched<SM, T, true, false, SINGLE>(p, s, t, pi, fhi_i, pos, p.fhi[lb], sx, sy, sz, es,
                                                               HELD::on ? cnt0 : -1, w0);
                 else
-                    steric_forces_batched<SM, T, false, false>(p, s, t, pi, fhi_i, pos, p.fhi[lb], sx, sy, sz, es);
+                    steric_forces_batched<SM, T, false, false, SINGLE>(p, s, t, pi, fhi_i, pos, p.fhi[lb], sx, sy, sz, es);
             }
             else if (p.pl16)
                 steric_forces<SM, T, 0>(p, s, t, pi, fhi_i, pos, p.fhi[lb], sx, sy, sz, es);
@@ -1201,7 +1182,7 @@ __device__ __forceinline__ int particle_step(const Params &p, const int s, const
             fx = fmaf(sx, kf, fx);
             fy = fmaf(sy, kf, fy);
             fz = fmaf(sz, kf, fz);
-            e[1] = es * p.steric_scale;
+            e[1] = __fmul_rn(es, p.steric_scale);
         }
         // springs after the steric pairs: no spring sums are live across the steric loop
         if (p.spring_on)
@@ -1215,7 +1196,7 @@ __device__ __forceinline__ int particle_step(const Params &p, const int s, const
             fx = fmaf(sx, kf, fx);
             fy = fmaf(sy, kf, fy);
             fz = fmaf(sz, kf, fz);
-            e[0] = es * p.spring_scale;
+            e[0] = __fmul_rn(es, p.spring_scale);
         }
         if ((!SINGLE || !BS_COUL_WARP) && p.coulomb_on && (fi & PF_CHARGED))
         {
@@ -1224,7 +1205,7 @@ __device__ __forceinline__ int particle_step(const Params &p, const int s, const
             fx = fmaf(sx, p.k_elec_f, fx);
             fy = fmaf(sy, p.k_elec_f, fy);
             fz = fmaf(sz, p.k_elec_f, fz);
-            e[2] = es * p.k_elec_e;
+            e[2] = __fmul_rn(es, p.k_elec_e);
         }
         if (!LEAN && p.hydro_on && (fi & PF_HYDROPHOBIC))
         {
@@ -1234,7 +1215,7 @@ __device__ __forceinline__ int particle_step(const Params &p, const int s, const
             fx = fmaf(sx, kf, fx);
             fy = fmaf(sy, kf, fy);
             fz = fmaf(sz, kf, fz);
-            e[3] = es * p.k_hydro_e * p.hydro_scale;
+            e[3] = __fmul_rn(es * p.k_hydro_e, p.hydro_scale);
         }
     }
     constexpr bool kEnergy = MODE != MODE_STEP_PART;
@@ -1280,7 +1261,7 @@ __device__ __forceinline__ int particle_step(const Params &p, const int s, const
                 fx = fmaf(cx, p.k_elec_f, fx);
                 fy = fmaf(cy, p.k_elec_f, fy);
                 fz = fmaf(cz, p.k_elec_f, fz);
-                e[2] = ce * p.k_elec_e;
+                e[2] = __fmul_rn(ce, p.k_elec_e);
             }
         }
     }
@@ -1309,9 +1290,9 @@ __device__ __forceinline__ int particle_step(const Params &p, const int s, const
             // ---- viscosity (Particle.cpp:80-84) ----
             if (p.visc_on)
             {
-                fx -= v.x * p.visc;
-                fy -= v.y * p.visc;
-                fz -= v.z * p.visc;
+                fx = fmaf(-v.x, p.visc, fx);
+                fy = fmaf(-v.y, p.visc, fy);
+                fz = fmaf(-v.z, p.visc, fz);
             }
             const float4 ip = p.iprm[lb][s];
             // ---- IMPALA, flat membrane (imp.hpp:29-159, ForceField.cpp:62-88) ----
@@ -1321,15 +1302,15 @@ __device__ __forceinline__ int particle_step(const Params &p, const int s, const
             {
                 const float ex = expf(p.imp_alpha * (fabsf(pi.z) - p.imp_z0));
                 const float cz = 0.5f - 1.0f / (1.0f + ex);
-                const float gg = -ip.y * ip.z + kAlip * ip.y;
-                e[4] = p.imp_scale * gg * cz;
+                const float gg = fmaf(kAlip, ip.y, -__fmul_rn(ip.y, ip.z));
+                e[4] = __fmul_rn(p.imp_scale * gg, cz);
                 // dC/dz = alpha sign(z) e / (1 + e)^2, written without overflow
                 float dcz = pi.z != 0.0f ? p.imp_alpha / (ex + 2.0f + 1.0f / ex) : 0.0f;
                 if (pi.z < 0.0f)
                     dcz = -dcz;
                 if (!isfinite(dcz))
                     dcz = 0.0f;
-                fz -= p.imp_scale * (gg * dcz * p.k_imp_f);
+                fz = fmaf(-p.imp_scale, gg * dcz * p.k_imp_f, fz);
             }
             // ---- external force (SpringNetwork::setForce, SpringNetwork.cpp:438-442) ----
             if (ext_on)
@@ -1378,8 +1359,8 @@ __device__ __forceinline__ int particle_step(const Params &p, const int s, const
                     vy = __fadd_rn(vy, __fmul_rn(__fdiv_rn(fy, m), p.dt));
                     vz = __fadd_rn(vz, __fmul_rn(__fdiv_rn(fz, m), p.dt));
                 }
-                const float v2 = vx * vx + vy * vy + vz * vz;
-                e[5] = 0.5f * m * v2 * p.k_kin;
+                const float v2 = norm2(vx, vy, vz);
+                e[5] = __fmul_rn(0.5f * m * v2, p.k_kin);
                 float nx, ny, nz;
                 if (!LEAN && p.pos_lo[0])
                 {
@@ -1407,7 +1388,7 @@ __device__ __forceinline__ int particle_step(const Params &p, const int s, const
                     pend |= ST_NONFINITE;
                 const float4 b = p.pos_build[s];
                 const float ddx = nx - b.x, ddy = ny - b.y, ddz = nz - b.z;
-                if (ddx * ddx + ddy * ddy + ddz * ddz > p.half_skin2)
+                if (norm2(ddx, ddy, ddz) > p.half_skin2)
                     pend |= ST_STALE;
             }
         }

@@ -194,7 +194,7 @@ __device__ int rigid_body_step(const Params &p, const int b, const int sold)
             pend |= ST_NONFINITE;
         const float4 bp = p.pos_build[s];
         const float ddx = nx - bp.x, ddy = ny - bp.y, ddz = nz - bp.z;
-        if (ddx * ddx + ddy * ddy + ddz * ddz > p.half_skin2)
+        if (norm2(ddx, ddy, ddz) > p.half_skin2)
             pend |= ST_STALE;
     }
     return pend;
