@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(kAdjRunBlock, T == 4 ? 3 : 2) k_adj_run(Params
         to = from;
         from = now;
         if (k > 0)
-            met = grid_barrier(p.order_sync, static_cast<unsigned int>(count - k), 0) != 0;
+            met = grid_barrier(p, p.order_sync, static_cast<unsigned int>(count - k), 0) != 0;
     }
     if (!met)
     {

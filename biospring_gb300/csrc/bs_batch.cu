@@ -505,7 +505,7 @@ __global__ void __launch_bounds__(kBatchMaxBlock, 2) k_batch_run(Params p, int c
     auto meet = [&](int pend) -> bool {
         if (csize == 1)
             return __syncthreads_or(pend) != 0;
-        const int r = group_barrier(p.grp_arrive + cid, static_cast<unsigned int>(csize), ++gen, pend);
+        const int r = group_barrier(p.grp_arrive + cid, static_cast<unsigned int>(csize), ++gen, pend, p.barrier_polls);
         if (raised && rank == 0 && threadIdx.x == 0)
             atomicAnd(p.grp_arrive + cid, ~(1u << (30 + ((gen - 1u) & 1u))));
         raised = r == 2;

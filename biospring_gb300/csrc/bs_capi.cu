@@ -165,6 +165,13 @@ int cuda_fail(bs_sim *s, cudaError_t e, const char *what)
             return cuda_fail(s, e_, #call);                                                                            \
     } while (0)
 
+// A kernel whose blocks wait for one another gave a wait up: the state is between two steps, and the raised bit keeps
+// every later kernel off it.
+int barrier_fail(bs_sim *s)
+{
+    return fail(s, BS_E_TIMEOUT, "a wait between the blocks of a kernel timed out: set the handle up again");
+}
+
 void destroy_graph(bs_sim *s)
 {
     if (s->period_graph)
@@ -362,7 +369,7 @@ int rebuild_now(bs_sim *s)
         if (st & ST_NONFINITE)
             return fail(s, BS_E_NONFINITE, "non-finite particle position");
         if (st & ST_BARRIER)
-            return fail(s, BS_E_CUDA, "a grid barrier of the step kernel timed out");
+            return barrier_fail(s);
         if (st & ST_CELL_CAPACITY)
         {
             const long long need = s->ctl_host->ncells_needed;
@@ -1621,6 +1628,9 @@ int bs_setup(bs_sim *s, const bs_config *cfg)
     p.k_imp_f = static_cast<float>(kImpForceConvert);
     p.k_hydro_e = static_cast<float>(kAvogadro * 1.0E-3);
 
+    p.barrier_polls = kBarrierPolls;
+    if (const char *env = std::getenv("BS_BARRIER_POLLS")) // shorter waits, for tests
+        p.barrier_polls = std::max(1, std::min(std::atoi(env), kBarrierPolls));
     BS_CUDA(load_step_kernels());
     BS_CUDA(order_blocks(p, &p.order_blocks));
     BS_CUDA(run_fits(p));
@@ -1728,7 +1738,7 @@ static int synchronize_batch(bs_sim *s)
                         "Found non-finite position in system " + std::to_string(first) + " of the batch");
         }
         if (h.status & ST_BARRIER)
-            return fail(s, BS_E_CUDA, "a barrier of the ensemble kernel timed out");
+            return barrier_fail(s);
         if (h.status & (ST_CELL_CAPACITY | ST_PAIR_CAPACITY | ST_WIDE))
         {
             rc = rebuild_now(s);
@@ -1773,7 +1783,7 @@ int bs_synchronize(bs_sim *s)
         if (h.status & ST_NONFINITE)
             return fail(s, BS_E_NONFINITE, "Found non-finite position (a particle position became NaN or infinite)");
         if (h.status & ST_BARRIER)
-            return fail(s, BS_E_CUDA, "a grid barrier of the step kernel timed out");
+            return barrier_fail(s);
         if (h.status & (ST_CELL_CAPACITY | ST_PAIR_CAPACITY | ST_WIDE))
         {
             rc = rebuild_now(s); // grows the lists and rebuilds
@@ -2641,7 +2651,7 @@ int bs_adjoint(bs_sim *s, int32_t nsteps, int32_t checkpoint, const float *targe
         if (h.status & ST_NONFINITE)
             return fail(s, BS_E_NONFINITE, "bs_adjoint: a position became non-finite");
         if (h.status & ST_BARRIER)
-            return fail(s, BS_E_CUDA, "bs_adjoint: a grid barrier timed out");
+            return barrier_fail(s);
         if ((h.status & ST_STALE) || h.stale_events != saved.stale_events)
         {
             // put the counters back before reporting

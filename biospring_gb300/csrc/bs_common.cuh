@@ -197,6 +197,7 @@ struct Params
     unsigned long long *cell_bin; // [cells][64] order keys by cell, where k_order takes the short way
     unsigned int *order_sync; // [3] k_order's grid-barrier word, finished blocks, full bin; 0 between launches
     int order_blocks;         // its grid, resident at once
+    int barrier_polls;        // polls after which a barrier between blocks gives up (ST_BARRIER)
     int pl_sparse;            // build the pair lists one warp per particle (few particles per cell)
     int lists_off;            // no nonbonded term is on: no pair lists, the grid only orders the particles
     int coul_all;             // list Coulomb partners of every dynamic particle, charged or not (charge gradients)

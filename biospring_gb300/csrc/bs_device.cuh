@@ -183,7 +183,7 @@ __device__ __forceinline__ bool pair_in(float r2, float lo2, float hi2, float4 p
 // Two flag bits, by the parity of gen: a block may already be at the next meeting when another reads
 // the word, but never two ahead.
 constexpr unsigned int kRunCount = (1u << 30) - 1u;
-__device__ __forceinline__ int group_barrier(unsigned int *arrive, unsigned int blocks, unsigned int gen, int pend)
+__device__ __forceinline__ int group_barrier(unsigned int *arrive, unsigned int blocks, unsigned int gen, int pend, int polls)
 {
     __shared__ int met;
     const int any = __syncthreads_or(pend);
@@ -197,16 +197,16 @@ __device__ __forceinline__ int group_barrier(unsigned int *arrive, unsigned int 
         int tries = 0;
         do
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(arrive) : "memory");
-        while ((seen & kRunCount) < want && ++tries < kRunSpinLimit);
+        while ((seen & kRunCount) < want && ++tries < polls);
         met = (seen & kRunCount) < want ? 0 : ((seen & flag) ? 2 : 1);
     }
     __syncthreads();
     return met;
 }
 
-__device__ __forceinline__ int grid_barrier(unsigned int *arrive, unsigned int gen, int pend)
+__device__ __forceinline__ int grid_barrier(const Params &p, unsigned int *arrive, unsigned int gen, int pend)
 {
-    return group_barrier(arrive, gridDim.x, gen, pend);
+    return group_barrier(arrive, gridDim.x, gen, pend, p.barrier_polls);
 }
 
 // Knuth's TwoSum: s = fl(a + b) and s + err == a + b exactly (round-to-nearest, no contraction).

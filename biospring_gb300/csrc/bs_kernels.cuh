@@ -100,10 +100,10 @@ const void *run_linear(int lanes, bool lean, int hold);
 const void *run_amber(int lanes, bool lean, int hold);
 const void *run_lewitt(int lanes, bool lean, int hold);
 const void *run_zacharias(int lanes, bool lean, int hold);
-// Steps of one launch (10 in the default schedule) and the polls after which a barrier gives up (some
-// seconds; a meeting takes about a microsecond).
+// Steps of one launch (10 in the default schedule) and the polls after which a barrier gives up (Params::
+// barrier_polls; some seconds, a meeting takes about a microsecond).
 constexpr int kRunMaxSteps = 1024;
-constexpr int kRunSpinLimit = 1 << 22;
+constexpr int kBarrierPolls = 1 << 22;
 // The lean step kernels leave out, at compile time, the terms most systems do not use (pairwise
 // hydrophobic forces, field grids, the probe, rigid bodies, float-float positions): fewer live
 // registers, so the common kernel runs without register spills.

@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(kOrderBlock, 4) k_order(Params p)
     const float4 *pos = p.pos[sb];
     unsigned int gen = 0;
     auto meet = [&]() {
-        const bool ok = grid_barrier(p.order_sync, ++gen, 0) != 0;
+        const bool ok = grid_barrier(p, p.order_sync, ++gen, 0) != 0;
         if (!ok && threadIdx.x == 0)
             atomicOr(&ctl->status, ST_BARRIER);
         return ok;

@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(kStepKernelBlock, HOLD ? HOLD : kStepMinBlocks
         }
         if (!LEAN && p.nbody > 0)
         {
-            if (!grid_barrier(p.run_arrive, ++gen, 0)) // the bodies read every member's force
+            if (!grid_barrier(p, p.run_arrive, ++gen, 0)) // the bodies read every member's force
             {
                 go = 0;
                 break;
@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(kStepKernelBlock, HOLD ? HOLD : kStepMinBlocks
         ++k;
         if (k < count || probe)
         {
-            go = grid_barrier(p.run_arrive, ++gen, pend);
+            go = grid_barrier(p, p.run_arrive, ++gen, pend);
             if (probe && go)
                 probe_step(p, part, prb, &probe_ke);
         }

@@ -34,7 +34,7 @@ extern "C" {
 #define BS_E_CUDA 2       /* a CUDA runtime call failed */
 #define BS_E_NONFINITE 3  /* non-finite position (reference: logging::die, SpringNetwork.cpp:222-229) */
 #define BS_E_CAPACITY 4   /* a device list overflowed and could not be regrown */
-#define BS_E_TIMEOUT 5    /* a bounded device-side wait gave up */
+#define BS_E_TIMEOUT 5    /* a bounded device-side wait gave up; the handle takes no step until bs_setup */
 #define BS_E_STATE 6      /* call made in the wrong order (e.g. step before setup) */
 
 /* ---- steric modes (steric.mode, src/configuration/Setting.hpp:269-273) ---------- */
@@ -258,7 +258,11 @@ int bs_setup(bs_sim *sim, const bs_config *cfg);
 int bs_step(bs_sim *sim, int32_t nsteps);
 
 /* Enqueues nsteps steps on the handle's stream and returns without waiting (the steps run as
- * captured CUDA graphs). Status is checked by the next synchronising call. */
+ * captured CUDA graphs). Status is checked by the next synchronising call. Several handles may be
+ * at work at once, from one thread or from a thread each; rebuilds, and the steps of systems of up
+ * to 38,912 particles, need all their blocks on the device together, so handles take turns there.
+ * Waits between the blocks of a kernel are bounded (some seconds): one that runs out gives
+ * BS_E_TIMEOUT from the next synchronising call on, until bs_setup. */
 int bs_step_async(bs_sim *sim, int32_t nsteps);
 
 /* Waits for enqueued work, checks the device status word and, if a particle drifted too far
