@@ -550,7 +550,8 @@ __global__ void k_adj_combine(int nsp, const float *gk, const float *gr0, float 
 
 int launch_adj_step(const Params &p, const AdjState &a, cudaStream_t st)
 {
-    // lanes per particle as in the forward step (smaller systems take k_adj_run)
+    // lanes per particle as in the forward step: 4 at the sizes that come here (smaller systems take k_adj_run), 8 or 2
+    // where BS_STEP_LANES says so
     const int T = p.step_lanes >= 8 ? 8 : (p.step_lanes == 2 ? 2 : 4);
     const int nb = static_cast<int>((static_cast<long long>(p.npad) * T + kStepBlock - 1) / kStepBlock);
     if (T == 8)

@@ -6,8 +6,9 @@
 // search grid (bounding box of its own particles, the single-system formula). Spring partners and
 // pair-list partners are always in the same system.
 //
-// Rebuild: k_order (bs_order.cu), then k_batch_pairlist (one warp per home particle: systems are
-// sparse, a cell holds a few particles).
+// Rebuild: k_order (bs_order.cu), then the pair lists: systems are sparse, a cell holds a few particles, so a home
+// particle is listed by one warp (k_batch_pairlist) or, in ensembles of 48,000 particles and more, by one thread
+// (k_home_pairlist).
 //
 // Step: k_batch_run, a persistent kernel, launched cooperatively. Its blocks form groups; a group owns
 // a list of whole systems (a host-side longest-processing-time assignment) and runs each of them for the

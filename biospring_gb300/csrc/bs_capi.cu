@@ -1588,10 +1588,11 @@ int bs_setup(bs_sim *s, const bs_config *cfg)
     p.imp_on = c.impala_enable != 0;
     p.visc_on = c.viscosity_enable != 0;
     p.steric_mode = c.steric_mode;
-    // lanes per particle: the fewest of 4, 8, 16 that still give the GPU some 64-80k threads
-    // (measured: 4 lanes from 20k particles, 8 from 8k, 16 below; 8 lanes end at 19,456, where 608 resident
-    // blocks hold the whole step and k_run takes it); BS_STEP_LANES overrides
-    p.step_lanes = n > 19456 ? 4 : (n >= 8000 ? 8 : 16);
+    // lanes per particle: the fewest of 4, 8, 16 that still give the GPU some 64-80k threads (measured: 4 lanes from 20k
+    // particles, 8 from 8k, 16 below; 8 lanes end where the resident blocks, kStepMinBlocks on each of 152 SMs, no longer
+    // hold the whole step, so that k_run takes it with 8 or with 4: 19,456 particles); BS_STEP_LANES overrides
+    constexpr int64_t kEightLanes = 152ll * kStepMinBlocks * kStepKernelBlock / 8;
+    p.step_lanes = n > kEightLanes ? 4 : (n >= 8000 ? 8 : 16);
     if (const char *env = std::getenv("BS_STEP_LANES"))
     {
         const int v = std::atoi(env);

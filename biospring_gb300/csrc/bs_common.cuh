@@ -198,7 +198,7 @@ struct Params
     unsigned int *order_sync; // [3] k_order's grid-barrier word, finished blocks, full bin; 0 between launches
     int order_blocks;         // its grid, resident at once
     int barrier_polls;        // polls after which a barrier between blocks gives up (ST_BARRIER)
-    int pl_sparse;            // build the pair lists one warp per particle (few particles per cell)
+    int pl_sparse;            // few particles per cell: the pair lists are built by a warp or a thread per particle
     int lists_off;            // no nonbonded term is on: no pair lists, the grid only orders the particles
     int coul_all;             // list Coulomb partners of every dynamic particle, charged or not (charge gradients)
     // energies: per-block partials
@@ -214,7 +214,7 @@ struct Params
     float dt;
     int spring_on, steric_on, coulomb_on, hydro_on, imp_on, visc_on;
     int steric_mode, dielectric_mode;
-    int step_lanes;           // threads per particle in the step kernel (1, 2, 4 or 8)
+    int step_lanes;           // threads per particle in the step kernel (2, 4, 8 or 16)
     float c_steric, c_coulomb, c_hydro;               // cutoffs
     float lo2_s, hi2_s, lo2_c, hi2_c, lo2_h, hi2_h;   // guard bands on r^2
     float list_radius;        // grid edge: largest cutoff + skin

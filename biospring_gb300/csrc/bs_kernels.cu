@@ -18,9 +18,11 @@
 // then needs only 1/r^2 (no square root, no division).
 //
 // Rebuild (every K steps, or when a particle drifted more than skin/2):
-//   k_order (bs_order.cu) -> k_pairlist (bs_list.cu), or k_batch_pairlist (bs_batch.cu) for sparse systems
+//   k_order (bs_order.cu) -> k_pairlist (bs_list.cu), or k_batch_pairlist or k_home_pairlist (bs_batch.cu) for sparse
+//   systems
 // Step: k_step, T consecutive lanes per particle, gathers its springs and nonbonded pairs (no
-// atomics on forces, so results are deterministic) and integrates in the same pass.
+// atomics on forces, so results are deterministic) and integrates in the same pass; where the grid is resident at
+// once k_run (bs_run.cuh) takes all steps up to the next rebuild.
 //
 // Reference behaviour reproduced (paths inside the BioSpring project):
 //   cell grid and cell id           src/nsearch.hpp:277-293, 342-390 (FP64, same formula; the

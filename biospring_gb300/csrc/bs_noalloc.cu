@@ -38,9 +38,7 @@ constexpr int kNaMaxN = BS_NOALLOC_MAX_PARTICLES;
 constexpr int kNaBlock = 256;                        // threads per block
 constexpr int kNaHomes = 4;                          // home particles of a warp
 constexpr int kNaMaxSplit = kNaBlock / 32;           // most warps that share a group of homes
-// most blocks of a call: 4, 8 and 16 homes a block up to 5,000, 10,000 and kNaMaxN particles
-// (na_split): at most 1,250
-constexpr int kNaMaxBlocks = 1280;
+constexpr int kNaMaxBlocks = 1280;                   // most blocks of a call (na_blocks)
 constexpr int kNaTerms = 3;                          // steric, Coulomb, hydrophobic
 
 // Scratch layout (byte offsets into na_scratch):
@@ -162,20 +160,6 @@ __global__ void __launch_bounds__(256) k_na_pack(NaParams p, const float *__rest
     b.prm[i] = make_float4(static_cast<float>(F), q, h, __uint_as_float(fl));
 }
 
-// All-pairs forces in two phases a warp. A warp owns kNaHomes home particles and runs through its
-// share of the particles j, 32 at a time, one a lane: phase 1 tests each against every home with the
-// FP32 squared distance alone and appends the accepted j to the home's queue (one ballot a home);
-// phase 2 takes a home's next 32 queued partners, one a lane, and evaluates every term. Within the
-// cutoffs of a dense system lie a few per cent of the particles, so evaluating in place would
-// run the pair body for one or two lanes of the warp in most windows; through the queue it runs
-// with all lanes busy, and the test, some 15 instructions for 32 pairs, is what bounds the kernel.
-// `split` warps (1, 2, 4 or 8) share a group of homes, each taking every split-th window, so that
-// small systems still fill the chip; the host picks it from n. The sums of the lanes and then
-// of the split warps are added in a fixed order.
-// Measured (pack and forces, us): one thread a particle in 64-thread blocks 139 / 798 / 2,285 at 500 /
-// 4,001 / 16,384 particles (63 blocks of 2 warps on 152 SMs at 4,001), this form 17 / 48 / 261. The
-// lanes' sums wait in shared memory: held in registers for four homes they took 118 of them, and
-// 16 warps an SM left 56% of the issue slots without a ready warp.
 // The pair terms of one home and one partner (steric.hpp, electrostatic.hpp, hydrophobic.hpp).
 __device__ __forceinline__ void na_pair(const NaParams &p, float4 pi, float4 qi, float4 pj, float4 qj, float (&v)[6])
 {
@@ -253,6 +237,20 @@ __device__ __forceinline__ void na_pair(const NaParams &p, float4 pi, float4 qi,
     fz = fmaf(dz, f, fz);
 }
 
+// All-pairs forces in two phases a warp. A warp owns kNaHomes home particles and runs through its
+// share of the particles j, 32 at a time, one a lane: phase 1 tests each against every home with the
+// FP32 squared distance alone and appends the accepted j to the home's queue (one ballot a home);
+// phase 2 takes a home's next 32 queued partners, one a lane, and evaluates every term. Within the
+// cutoffs of a dense system lie a few per cent of the particles, so evaluating in place would
+// run the pair body for one or two lanes of the warp in most windows; through the queue it runs
+// with all lanes busy, and the test, some 15 instructions for 32 pairs, is what bounds the kernel.
+// `split` warps (1, 2, 4 or 8) share a group of homes, each taking every split-th window, so that
+// small systems still fill the chip; the host picks it from n. The sums of the lanes and then
+// of the split warps are added in a fixed order.
+// Measured (pack and forces, us): one thread a particle in 64-thread blocks 139 / 798 / 2,285 at 500 /
+// 4,001 / 16,384 particles (63 blocks of 2 warps on 152 SMs at 4,001), this form 17 / 44 / 260. The
+// lanes' sums wait in shared memory: held in registers for four homes they took 118 of them, and
+// 16 warps an SM left 56% of the issue slots without a ready warp.
 __global__ void __launch_bounds__(kNaBlock, 3) k_na_forces(NaParams p, int split, float *__restrict__ forces,
                                                         double *__restrict__ energies, NaBuffers b)
 {
@@ -480,12 +478,18 @@ __global__ void __launch_bounds__(kNaBlock, 3) k_na_forces(NaParams p, int split
         *b.done = 0u; // ready for the next call
 }
 
-// Warps that share a group of homes: some 8,000 warps up to 10,000 particles (four times what the
-// chip holds at once), so that the last blocks to finish are short; half as many homes a block cost
-// more in part-filled queues than they gain. Measured (us a call, 2,500 / 5,000 / 10,000 / 16,384
-// particles): this rule 31 / 56 / 124 / 261; a warp for every group from 10,000 and half the split
-// below 31 / 54 / 129 / 307; the split halved again 29 / 57 / 156 / 307.
-int na_split(int n) { return n <= 5000 ? 8 : (n <= 10000 ? 4 : 2); }
+// Warps that share a group of homes: 2 n warps up to 5,000 particles, n up to 10,000, n / 2 above, so 8,000 to 10,000
+// at the upper ends (more than twice what the chip holds at once), so that the last blocks to finish are short; half as
+// many homes a block cost more in part-filled queues than they gain. Measured (us a call, 2,500 / 5,000 / 10,000 /
+// 16,384 particles): this rule 29 / 51 / 123 / 260, half the split 29 / 52 / 130 / 307.
+constexpr int na_split(int n) { return n <= 5000 ? 8 : (n <= 10000 ? 4 : 2); }
+constexpr int na_blocks(int n)
+{
+    const int homes = kNaHomes * (kNaMaxSplit / na_split(n));
+    return (n + homes - 1) / homes;
+}
+static_assert(na_blocks(5000) <= kNaMaxBlocks && na_blocks(10000) <= kNaMaxBlocks && na_blocks(kNaMaxN) <= kNaMaxBlocks,
+              "energy partials for every block");
 
 float na_band_lo2(double c) { return static_cast<float>((c * (1.0 - 1.0 / 16384.0)) * (c * (1.0 - 1.0 / 16384.0))); }
 float na_band_hi2(double c) { return static_cast<float>((c * (1.0 + 1.0 / 16384.0)) * (c * (1.0 + 1.0 / 16384.0))); }
@@ -631,9 +635,9 @@ extern "C" int bs_nonbonded_forces_noalloc(const bs_config *cfg, int64_t n, cons
     k_na_pack<<<(p.n + 255) / 256, 256, 0, st>>>(p, d_xyz, d_radius, d_epsilon, d_charge, d_hydrophobicity,
                                                   d_is_static, b);
     // the force kernel starts launching while the packing runs and waits for it on the device
-    const int split = na_split(p.n), per_block = kNaHomes * (kNaMaxSplit / split);
+    const int split = na_split(p.n);
     cudaLaunchConfig_t lc{};
-    lc.gridDim = dim3((p.n + per_block - 1) / per_block);
+    lc.gridDim = dim3(na_blocks(p.n));
     lc.blockDim = dim3(kNaBlock);
     lc.stream = st;
     cudaLaunchAttribute attr[1];
