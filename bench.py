@@ -59,7 +59,7 @@ CTL_BYTES = 272                       # device control block (status, step count
 # DRAM bytes (read + write) of one k_step launch on this workload after an L2 flush, from one ncu
 # capture of dram__bytes_read.sum + dram__bytes_write.sum, and the digest of the step kernel's
 # sources that capture ran on: when the sources have changed since, the line marks the figure stale.
-STEP_KERNEL_TRAFFIC = {"bytes": 69.4976e6 + 1.227776e6, "sources_sha": "3ae85b626f5e23a6", "captured": "2026-12-05"}
+STEP_KERNEL_TRAFFIC = {"bytes": 69.495296e6 + 1.171712e6, "sources_sha": "748faa03ad384dea", "captured": "2026-12-05"}
 STEP_KERNEL_SOURCES = ("biospring_gb300/csrc/bs_device.cuh", "biospring_gb300/csrc/bs_kernels.cu",
                        "biospring_gb300/csrc/bs_kernels.cuh", "biospring_gb300/csrc/bs_common.cuh")
 DIELECTRIC_NOTE = ("Coulomb eps = 4r (distance-dependent), as the 100k configuration states; the reference's "

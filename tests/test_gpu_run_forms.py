@@ -81,3 +81,23 @@ def test_list_goes_stale_within_a_period():
         if k == 4:  # half a period: the list was stale before its rebuild was due
             assert np.linalg.norm(b.getPositions() - s.xyz, axis=1).max() > 0.3
     _same(a, b, 37)
+
+
+@pytest.mark.parametrize("extra", ["none", "hydrophobic", "bodies", "probe"])
+@pytest.mark.parametrize("n", [300, 5000, 10000, 20000])
+def test_one_step_a_call(n, extra):
+    """A call of one step takes the single-step kernel, with bodies or the probe the kernel of several."""
+    s = _beads(n, 1, extra == "hydrophobic")
+    if extra == "bodies":
+        free = np.flatnonzero(s.is_static == 0)
+        s.bodies = [free[k:k + 50].astype(np.int32) for k in (0, 150)]
+        s.config.update(rigidbody_enable=1, timestep=0.002)
+    if extra == "probe":
+        s.config.update(probe_enable=1, probe_steric=1, probe_electrostatic=1, probe_x=-4.0, probe_y=10.0, probe_z=10.0,
+                        probe_mass=70.0, probe_epsilon=0.5, probe_radius=3.0, probe_charge=1.0)
+    a, b = gpu_network(s), gpu_network(s)
+    a.computeStep(14)
+    for _ in range(14):
+        b.computeStep(1)
+    assert np.array_equal(a.getProbe(), b.getProbe())
+    _same(a, b, 14)
